@@ -60,6 +60,40 @@ def test_conv3x3_forward_and_gradients_match_torch(B, Cin, Cout, H, W):
     assert _rel(db, br.grad) < 1e-4
 
 
+# tile edges of the implicit GEMM: rows around the 128- and 256-pixel tiles (one band of pixels or three
+# segments), one and two pixel tiles per CTA, 16/32/64 output channels, channels that are no multiple
+# of 8, 16 or 32, and clusters that share the input channels unevenly
+@pytest.mark.parametrize("B,Cin,Cout,H,W", [(1, 40, 24, 3, 127), (1, 33, 40, 2, 130), (1, 16, 70, 1, 257), (2, 4, 3, 3, 600),
+                                             (1, 300, 33, 4, 9), (1, 96, 256, 4, 4), (3, 1, 1, 1, 1), (20, 8, 40, 64, 64),
+                                             (20, 9, 2, 64, 63), (20, 40, 32, 63, 64), (2, 130, 64, 5, 129)])
+def test_conv3x3_at_tile_edges(B, Cin, Cout, H, W):
+    test_conv3x3_forward_and_gradients_match_torch(B, Cin, Cout, H, W)
+
+
+def test_weight_gradient_with_infinite_and_nan_inputs():
+    """An infinity or NaN at an image's edge reaches only the taps whose products it is part of (the
+    zeros of the padding times the gradient, never the input times a gradient outside the image)."""
+    torch = pytest.importorskip("torch")
+    lib = capi.load()
+    B, Cin, Cout, H, W = 2, 3, 4, 5, 6
+    g = torch.Generator().manual_seed(9)
+    x = torch.randn(B, Cin, H, W, generator=g)
+    x[0, 0, 0, 0], x[1, 1, H - 1, W - 1] = float("inf"), float("nan")
+    d = 1 + torch.rand(B, Cout, H, W, generator=g)
+    x, d = x.to(torch.bfloat16), d.to(torch.bfloat16)
+    cols = torch.nn.functional.unfold(x.double(), 3, padding=1).reshape(B, Cin, 9, H * W)
+    ref = torch.einsum("boq,bctq->oct", d.double().reshape(B, Cout, H * W), cols).reshape(Cout, Cin, 3, 3)
+    xd, dd = x.cuda(), d.cuda()
+    dw = torch.empty(Cout, Cin, 3, 3, device="cuda")
+    db = torch.empty(Cout, device="cuda")
+    capi.check(lib.mt_sg_conv3x3_backward_weight(_p(xd), _p(dd), None, _p(dw), _p(db), B, Cin, Cout, H, W, None))
+    dw = dw.cpu().double()
+    assert torch.equal(dw.isnan(), ref.isnan()) and torch.equal(dw.isinf(), ref.isinf())
+    ok = ref.isfinite()
+    assert ok.any() and not ok.all()
+    assert _rel(dw[ok], ref[ok]) < 1e-4
+
+
 def test_loss_and_adam_match_their_formulas():
     torch = pytest.importorskip("torch")
     lib = capi.load()
