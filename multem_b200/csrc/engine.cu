@@ -911,25 +911,25 @@ void Engine::run_conf_batch(ConfData* const* cds, int nb) {
         if (cds[b]->n_slice != cds[0]->n_slice || cds[b]->last_slice != cds[0]->last_slice ||
             cds[b]->slice_ithk != cds[0]->slice_ithk)
             fail(MT_ERR_INTERNAL, "configurations of a batch must share their slicing");
-    for (int b = 0; b < nb; b++) {
-        const ConfData& cd = *cds[b];
-        float2* trans = d_trans_.p + b * tstride;
-        // transmission functions of the slices up to the last output thickness
+    // transmission functions of the slices up to the last output thickness, several configurations
+    // per launch
+    for (int b0 = 0; b0 < nb; b0 += kSplatConfs) {
         SplatArgs sa{};
         sa.g = gdev_;
-        sa.atoms = cd.atoms.p;
-        sa.slice_range = cd.ranges.p;
+        sa.n_conf = std::min(kSplatConfs, nb - b0);
+        for (int b = 0; b < sa.n_conf; b++) sa.conf[b] = {cds[b0 + b]->atoms.p, cds[b0 + b]->ranges.p};
+        sa.trans_stride = tstride;
         sa.tab = d_tab_.p;
         sa.R_max = d_Rmax_.p;
         sa.n_types = (int)Z_of_type_.size();
         sa.nR = m_.nR;
         sa.w = m_.Vr_factor();
         sa.wpo = (m_.interaction_model == 3);
-        sa.trans = trans;
-        sa.V = nullptr;
-        launch_splat(sa, 0, cd.last_slice + 1, stream_);
-        if (d_bwl_.p) band_limit_trans(cd, trans);
+        sa.trans = d_trans_.p + b0 * tstride;
+        launch_splat(sa, 0, cds[0]->last_slice + 1, stream_);
     }
+    if (d_bwl_.p)
+        for (int b = 0; b < nb; b++) band_limit_trans(*cds[b], d_trans_.p + b * tstride);
     if (m_.is_scanning()) run_stem(*cds[0]); else run_ew(cds, nb);
 }
 
@@ -1525,8 +1525,8 @@ void Engine::projected_potential(int iconf, int islice, double* V, double* trans
     dT.alloc(nxy);
     SplatArgs sa{};
     sa.g = gdev_;
-    sa.atoms = cd.atoms.p;
-    sa.slice_range = cd.ranges.p + islice;
+    sa.n_conf = 1;
+    sa.conf[0] = {cd.atoms.p, cd.ranges.p + islice};
     sa.tab = d_tab_.p;
     sa.R_max = d_Rmax_.p;
     sa.n_types = (int)Z_of_type_.size();

@@ -56,19 +56,26 @@ void encode_tile_map(CUtensorMap* map, const float2* base, int nx, int ldy, int 
 // of a slice and every pixel of its footprint box (get_bn, src/cpu_fcns.hpp:1670-1684),
 //   R2 = (ix*dRx + Rx_0 - x)^2 + (iy*dRy + Ry_0 - y)^2;  if R2 < R2_max:
 //   V[ind_col_pbc_shift(ix, iy)] += occ * cubic(R2)   (eval_cubic_poly, src/cgpu_fcns.cuh:1498-1567)
-// with an FP32 atomicAdd per contribution. Here one CTA owns a 64 x 32 tile of the stored
-// (shifted) grid of one slice (8 pixels per thread, 8 rows apart), culls the slice's atoms against
-// its tile, and sums the contributions of the surviving atoms in atom order in registers
-// (deterministic, no atomics; the tile size changes no sum).
-// The epilogue writes T = exp(i*w*V) (functor::transmission_function, src/cgpu_fcns.cuh:3072-3086)
-// directly; V never goes to HBM unless asked for. Float products and sums use the _rn intrinsics
-// so they are not fused into FMAs and round like the reference's host float path.
+// with an FP32 atomicAdd per contribution. Here one CTA owns a tile of 8*PX x 32 pixels of the stored
+// (shifted) grid of one slice of one configuration, culls the slice's atoms against its tile, and
+// sums the contributions of the surviving atoms in atom order in registers (deterministic, no atomics;
+// the tile size changes no sum). The epilogue writes T = exp(i*w*V) (functor::transmission_function,
+// src/cgpu_fcns.cuh:3072-3086) directly; V never goes to HBM unless asked for. Float products and sums
+// use the _rn intrinsics so they are not fused into FMAs and round like the reference's host float path.
+//
+// Bound by instructions. A warp owns PX consecutive x of 32 consecutive y: (x - x_atom)^2 is the same
+// for its 32 lanes, so an atom whose circle does not reach a row of the warp costs that row one
+// uniform test, and (y - y_atom)^2 is computed once per atom; about 0.6 of the pixels visited lie inside
+// the circle (0.17 when each thread's pixels were spread over the whole tile). Two pixels are
+// evaluated together with packed sums and products (the same roundings), their spline interval found
+// from a base-2 logarithm and two exact comparisons with one 8-byte load, the four coefficients from
+// one 16-byte load; about 25 issue cycles per warp and evaluation. Measured on one B200 per
+// configuration: Si 256^2 x 32 slices 54 -> 26 us (eight configurations in one launch), SrTiO3 512^2 x
+// 50 slices 546 -> 325 us, 128^2 x 16 slices 47 -> 15 us, Au(110) 2048^2 x 30 slices 1745 -> 1129 us.
 // =============================================================================================
-constexpr int SPLAT_TX = 64;   // tile extent along x (slow index)
-constexpr int SPLAT_PX = SPLAT_TX / 8;  // pixels per thread along x
-constexpr int SPLAT_TY = 32;   // tile extent along y (contiguous index)
+constexpr int SPLAT_TY = 32;   // tile extent along y (contiguous index): one per lane
 constexpr int SPLAT_THREADS = 256;
-constexpr int SPLAT_MAXT_SMEM = 8;
+constexpr int SPLAT_WARPS = SPLAT_THREADS / 32;
 
 __device__ __forceinline__ int pmod(int a, int n) {
     int r = a % n;
@@ -76,47 +83,89 @@ __device__ __forceinline__ int pmod(int a, int n) {
 }
 
 struct AtomFoot {
-    float x, y, occ;
-    int type;
+    float x, y, occ, R2_max;
     int ix0, nxa, iy0, nya;
     int sx, sy;  // first footprint pixel in stored (shifted) coordinates
+    int type, pad;
 };
 
-__global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int islice_0) {
-    extern __shared__ float sm_tab[];
+// Spline tables in shared memory: per type nR knot pairs (R2[i], R2[i+1]) and coefficients (c0..c3)[i].
+struct SplatTables {
+    const float2* knot;
+    const float4* coef;
+    int nR;
+};
+
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// The interval of unrolledBinarySearch_c_nR (src/cgpu_fcns.cuh:1498-1518): the largest i in [0, nR-2]
+// with knot[i] <= R2 (0 below the first knot). The knots are log-spaced in R, so the guess is linear in
+// log2(R2); exact comparisons decide. Returns knot[i].
+__device__ __forceinline__ float spline_interval(const float2* knot, int nR, float scale, float offset, float R2, int& i) {
+    // floor of a value in [0.5, nR - 2] through the rounding of a sum with 2^23 - 0.5
+    const float g = fminf(fmaxf(__fmaf_rn(__log2f(R2), scale, offset), 0.5f), (float)(nR - 2));
+    i = __float_as_int(__fadd_rn(g, 8388607.5f)) - 0x4B000000;
+    float2 k = knot[i];
+    while (i > 0 && R2 < k.x) k = knot[--i];
+    while (i < nR - 2 && !(R2 < k.y)) k = knot[++i];
+    return k.x;
+}
+
+template <int PX>
+__global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int islice_0, int n_slice) {
+    extern __shared__ float4 sm_coef[];  // n_types * nR coefficients, then the knot pairs
     __shared__ AtomFoot s_list[SPLAT_THREADS];
-    __shared__ int s_warp_cnt[SPLAT_THREADS / 32];
-    __shared__ int s_n;
+    __shared__ int s_warp_cnt[SPLAT_WARPS];
+    __shared__ float2 s_guess[kMaxTypes];  // log2(R2) -> interval: scale, offset
+    constexpr int TX = SPLAT_WARPS * PX;
 
     const int nR = a.nR;
-    const int ntab = (a.n_types <= SPLAT_MAXT_SMEM) ? a.n_types : 0;
-    for (int i = threadIdx.x; i < ntab * 5 * nR; i += blockDim.x) sm_tab[i] = a.tab[i];
-    const float* tab = (ntab > 0) ? sm_tab : a.tab;
+    float2* sm_knot = reinterpret_cast<float2*>(sm_coef + a.n_types * nR);
+    for (int i = threadIdx.x; i < a.n_types * nR; i += SPLAT_THREADS) {
+        const int type = i / nR, k = i - type * nR;
+        const float* T = a.tab + (size_t)type * 5 * nR;
+        sm_coef[i] = make_float4(T[nR + k], T[2 * nR + k], T[3 * nR + k], T[4 * nR + k]);
+        sm_knot[i] = make_float2(T[k], T[k + 1 < nR ? k + 1 : k]);
+        if (k == 0) {
+            const float lg0 = __log2f(T[0]), scale = (float)(nR - 1) / (__log2f(T[nR - 1]) - lg0);
+            s_guess[type] = make_float2(scale, -lg0 * scale);
+        }
+    }
 
     const GridDev g = a.g;
-    const int islice = islice_0 + blockIdx.z;
-    const int tx0 = blockIdx.y * SPLAT_TX;
+    const int iconf = blockIdx.z / n_slice, islice = islice_0 + blockIdx.z % n_slice;
+    const float4* atoms = a.conf[iconf].atoms;
+    const int2 rng = a.conf[iconf].slice_range[islice];
+    const int tx0 = blockIdx.y * TX;
     const int ty0 = blockIdx.x * SPLAT_TY;
-    const int ly = threadIdx.x % SPLAT_TY;
-    const int lx = threadIdx.x / SPLAT_TY;  // 0..7: this thread's pixels are tx0 + lx + 8p
-    const int jy = ty0 + ly;
-    float V[SPLAT_PX];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int jy = ty0 + lane, jx0 = tx0 + warp * PX;  // this thread's pixels: (jx0 + p, jy)
+    unsigned long long V[PX / 2];  // pixels (2q, 2q + 1)
 #pragma unroll
-    for (int p = 0; p < SPLAT_PX; p++) V[p] = 0.0f;
+    for (int q = 0; q < PX / 2; q++) V[q] = 0ull;
 
-    const int2 rng = a.slice_range[islice];
     __syncthreads();
     for (int c0 = rng.x; c0 <= rng.y; c0 += SPLAT_THREADS) {
         const int ia = c0 + threadIdx.x;
         AtomFoot f;
         bool hit = false;
         if (ia <= rng.y) {
-            float4 at = a.atoms[ia];
+            float4 at = atoms[ia];
             f.x = at.x;
             f.y = at.y;
             f.occ = at.z;
             f.type = __float_as_int(at.w);
             const float Rm = a.R_max[f.type];
+            f.R2_max = __fmul_rn(Rm, Rm);
             // get_bn (src/cpu_fcns.hpp:1670-1684), periodic
             int i0 = (int)floorf(__fdiv_rn(__fsub_rn(f.x, Rm), g.dRx));
             int ie = (int)ceilf(__fdiv_rn(__fadd_rn(f.x, Rm), g.dRx));
@@ -129,65 +178,86 @@ __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int i
             f.sx = (pmod(f.ix0, g.nx) + g.nxh) % g.nx;
             f.sy = (pmod(f.iy0, g.ny) + g.nyh) % g.ny;
             // circular overlap of [sx, sx+nxa) with [tx0, tx0+TX) (and y)
-            bool ox = (f.nxa >= g.nx) || (pmod(tx0 - f.sx, g.nx) < f.nxa) || (pmod(f.sx - tx0, g.nx) < SPLAT_TX);
+            bool ox = (f.nxa >= g.nx) || (pmod(tx0 - f.sx, g.nx) < f.nxa) || (pmod(f.sx - tx0, g.nx) < TX);
             bool oy = (f.nya >= g.ny) || (pmod(ty0 - f.sy, g.ny) < f.nya) || (pmod(f.sy - ty0, g.ny) < SPLAT_TY);
             hit = ox && oy && f.nxa > 0 && f.nya > 0;
         }
         // deterministic compaction in atom order
         const unsigned m = __ballot_sync(0xffffffffu, hit);
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         if (lane == 0) s_warp_cnt[warp] = __popc(m);
         __syncthreads();
-        if (threadIdx.x == 0) {
-            int acc = 0;
-            for (int w = 0; w < SPLAT_THREADS / 32; w++) {
-                int cnt = s_warp_cnt[w];
-                s_warp_cnt[w] = acc;
-                acc += cnt;
-            }
-            s_n = acc;
+        int n = 0, first = 0;
+#pragma unroll
+        for (int w = 0; w < SPLAT_WARPS; w++) {
+            if (w == warp) first = n;
+            n += s_warp_cnt[w];
         }
+        if (hit) s_list[first + __popc(m & ((1u << lane) - 1u))] = f;
         __syncthreads();
-        if (hit) s_list[s_warp_cnt[warp] + __popc(m & ((1u << lane) - 1u))] = f;
-        __syncthreads();
-        const int n = s_n;
         for (int k = 0; k < n; k++) {
             const AtomFoot af = s_list[k];
-            const float* T = tab + (size_t)af.type * 5 * nR;
-            const float Rm = a.R_max[af.type];
-            const float R2_max = __fmul_rn(Rm, Rm);
-            // knot index guess: the knots are log-spaced in R, so log2(R^2) is linear in the index
-            const float lg0 = __log2f(T[0]);
-            const float lgs = (float)(nR - 1) / (__log2f(T[nR - 1]) - lg0);
-            // y offset, shared by every pixel of this thread (jy and sy are both in [0, ny))
+            const float2* knot = sm_knot + af.type * nR;
+            const float4* coef = sm_coef + af.type * nR;
+            const float2 guess = s_guess[af.type];
+            // offset in the footprint, of the first periodic image (jy and sy are both in [0, ny))
             int offy = jy - af.sy;
             if (offy < 0) offy += g.ny;
+            if (af.nxa <= g.nx && af.nya <= g.ny) {  // at most one image of the footprint at each pixel
+                const float Ry = __fsub_rn(__fadd_rn(__fmul_rn((float)(af.iy0 + offy), g.dRy), g.Ry_0), af.y);
+                const float Ry2 = __fmul_rn(Ry, Ry);
+                const bool iny = offy < af.nya && Ry2 < af.R2_max;
+                if (!__any_sync(0xffffffffu, iny)) continue;
+                const unsigned long long occ = pack2(make_float2(af.occ, af.occ));
 #pragma unroll
-            for (int p = 0; p < SPLAT_PX; p++) {
-                const int jx = tx0 + lx + 8 * p;
-                int offx = jx - af.sx;
-                if (offx < 0) offx += g.nx;
-                for (int ox = offx; ox < af.nxa; ox += g.nx) {
-                    const int ix = af.ix0 + ox;
-                    const float Rx = __fsub_rn(__fadd_rn(__fmul_rn((float)ix, g.dRx), g.Rx_0), af.x);
-                    for (int oy = offy; oy < af.nya; oy += g.ny) {
-                        const int iy = af.iy0 + oy;
-                        const float Ry = __fsub_rn(__fadd_rn(__fmul_rn((float)iy, g.dRy), g.Ry_0), af.y);
-                        const float R2 = __fadd_rn(__fmul_rn(Rx, Rx), __fmul_rn(Ry, Ry));
-                        if (R2 < R2_max) {
-                            // the interval of unrolledBinarySearch_c_nR (src/cgpu_fcns.cuh:1498-1518):
-                            // the largest i0 in [0, nR-2] with T[i0] <= R2 (0 below the first knot),
-                            // from the logarithmic guess and exact comparisons with the knots
-                            int i0 = (int)fminf(fmaxf(__fmul_rn(__log2f(R2) - lg0, lgs), 0.0f), (float)(nR - 2));
-                            while (i0 > 0 && R2 < T[i0]) i0--;
-                            while (i0 < nR - 2 && !(R2 < T[i0 + 1])) i0++;
-                            const float dx = __fsub_rn(R2, T[i0]);
-                            const float c3 = T[4 * nR + i0], c2 = T[3 * nR + i0], c1 = T[2 * nR + i0], c0v = T[nR + i0];
-                            float v = __fadd_rn(__fmul_rn(c3, dx), c2);
-                            v = __fadd_rn(__fmul_rn(v, dx), c1);
-                            v = __fadd_rn(__fmul_rn(v, dx), c0v);
-                            v = __fmul_rn(af.occ, v);
-                            V[p] += v;
+                for (int q = 0; q < PX / 2; q++) {
+                    float R2[2];
+                    bool in[2];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        int offx = jx0 + 2 * q + h - af.sx;
+                        if (offx < 0) offx += g.nx;
+                        const float Rx = __fsub_rn(__fadd_rn(__fmul_rn((float)(af.ix0 + offx), g.dRx), g.Rx_0), af.x);
+                        const float Rx2 = __fmul_rn(Rx, Rx);
+                        R2[h] = __fadd_rn(Rx2, Ry2);
+                        in[h] = offx < af.nxa && Rx2 < af.R2_max;  // the same for every lane
+                    }
+                    if (!in[0] && !in[1]) continue;
+                    in[0] = in[0] && iny && R2[0] < af.R2_max;
+                    in[1] = in[1] && iny && R2[1] < af.R2_max;
+                    if (!in[0] && !in[1]) continue;
+                    int i0, i1;
+                    const float d0 = __fsub_rn(R2[0], spline_interval(knot, nR, guess.x, guess.y, R2[0], i0));
+                    const float d1 = __fsub_rn(R2[1], spline_interval(knot, nR, guess.x, guess.y, R2[1], i1));
+                    const float4 e0 = coef[i0], e1 = coef[i1];
+                    const unsigned long long d = pack2(make_float2(d0, d1));
+                    unsigned long long v = add2(mul2(pack2(make_float2(e0.w, e1.w)), d), pack2(make_float2(e0.z, e1.z)));
+                    v = add2(mul2(v, d), pack2(make_float2(e0.y, e1.y)));
+                    v = add2(mul2(v, d), pack2(make_float2(e0.x, e1.x)));
+                    const float2 r = unpack2(mul2(occ, v));
+                    V[q] = add2(V[q], pack2(make_float2(in[0] ? r.x : 0.0f, in[1] ? r.y : 0.0f)));
+                }
+            } else {  // a footprint wider than the grid: every image in order
+#pragma unroll
+                for (int p = 0; p < PX; p++) {
+                    int offx = jx0 + p - af.sx;
+                    if (offx < 0) offx += g.nx;
+                    for (int ox = offx; ox < af.nxa; ox += g.nx) {
+                        const float Rx = __fsub_rn(__fadd_rn(__fmul_rn((float)(af.ix0 + ox), g.dRx), g.Rx_0), af.x);
+                        for (int oy = offy; oy < af.nya; oy += g.ny) {
+                            const float Ry = __fsub_rn(__fadd_rn(__fmul_rn((float)(af.iy0 + oy), g.dRy), g.Ry_0), af.y);
+                            const float R2 = __fadd_rn(__fmul_rn(Rx, Rx), __fmul_rn(Ry, Ry));
+                            if (R2 < af.R2_max) {
+                                int i;
+                                const float dx = __fsub_rn(R2, spline_interval(knot, nR, guess.x, guess.y, R2, i));
+                                const float4 e = coef[i];
+                                float v = __fadd_rn(__fmul_rn(e.w, dx), e.z);
+                                v = __fadd_rn(__fmul_rn(v, dx), e.y);
+                                v = __fadd_rn(__fmul_rn(v, dx), e.x);
+                                v = __fmul_rn(af.occ, v);
+                                float2 s = unpack2(V[p / 2]);
+                                (p % 2 ? s.y : s.x) += v;
+                                V[p / 2] = pack2(s);
+                            }
                         }
                     }
                 }
@@ -195,14 +265,15 @@ __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int i
         }
         __syncthreads();
     }
-    const size_t base = (size_t)islice * g.nx * g.ny;
+    const size_t base = (size_t)iconf * a.trans_stride + (size_t)islice * g.nx * g.ny;
 #pragma unroll
-    for (int p = 0; p < SPLAT_PX; p++) {
-        const int jx = tx0 + lx + 8 * p;
-        const size_t idx = base + (size_t)jx * g.ny + jy;
-        if (a.V) a.V[idx] = V[p];
+    for (int p = 0; p < PX; p++) {
+        const size_t idx = base + (size_t)(jx0 + p) * g.ny + jy;
+        const float2 s = unpack2(V[p / 2]);
+        const float v = p % 2 ? s.y : s.x;
+        if (a.V) a.V[idx] = v;
         if (a.trans) {
-            const float th = __fmul_rn(a.w, V[p]);
+            const float th = __fmul_rn(a.w, v);
             float sn, cs;
             if (a.wpo) {
                 cs = 1.0f;
@@ -215,13 +286,25 @@ __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int i
     }
 }
 
-void launch_splat(const SplatArgs& a, int islice_0, int n_slice, cudaStream_t s) {
-    if (a.g.nx % SPLAT_TX || a.g.ny % SPLAT_TY) fail(MT_ERR_UNSUPPORTED, "grid must be a multiple of 64 x 32");
-    dim3 grid(a.g.ny / SPLAT_TY, a.g.nx / SPLAT_TX, n_slice);
-    size_t sm = (a.n_types <= SPLAT_MAXT_SMEM) ? (size_t)a.n_types * 5 * a.nR * sizeof(float) : 0;
-    splat_kernel<<<grid, SPLAT_THREADS, sm, s>>>(a, islice_0);
+template <int PX>
+static void splat_launch(const SplatArgs& a, int islice_0, int n_slice, cudaStream_t s) {
+    const dim3 grid(a.g.ny / SPLAT_TY, a.g.nx / (SPLAT_WARPS * PX), n_slice * a.n_conf);
+    const size_t sm = (size_t)a.n_types * a.nR * (sizeof(float4) + sizeof(float2));
+    MTB_CUDA(cudaFuncSetAttribute(splat_kernel<PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    splat_kernel<PX><<<grid, SPLAT_THREADS, sm, s>>>(a, islice_0, n_slice);
     g_launches++;
     MTB_CUDA(cudaGetLastError());
+}
+
+// Slices islice_0 .. islice_0 + n_slice - 1 of the n_conf configurations of `a` in one launch. Taller
+// warps (more pixels per thread) reuse a lane's (y - y_atom)^2 more often; shorter ones where the tiles
+// would leave an SM with less than four CTAs.
+void launch_splat(const SplatArgs& a, int islice_0, int n_slice, cudaStream_t s) {
+    if (a.g.nx % (SPLAT_WARPS * 8) || a.g.ny % SPLAT_TY) fail(MT_ERR_UNSUPPORTED, "grid must be a multiple of 64 x 32");
+    const long long tiles = (long long)(a.g.nx / 64) * (a.g.ny / SPLAT_TY) * n_slice * a.n_conf;
+    if (tiles >= 4 * 148) splat_launch<8>(a, islice_0, n_slice, s);
+    else if (2 * tiles >= 4 * 148) splat_launch<4>(a, islice_0, n_slice, s);
+    else splat_launch<2>(a, islice_0, n_slice, s);
 }
 
 // =============================================================================================

@@ -17,18 +17,24 @@ struct GridDev {
 };
 
 // ---- projected potential + transmission (splat) ----
-struct SplatArgs {
-    GridDev g;
+constexpr int kSplatConfs = 8;  // configurations per launch
+struct SplatConf {
     const float4* atoms;       // (x, y, occ, type index as int bits), z-sorted
     const int2* slice_range;   // per slice (iatom_0, iatom_e), empty when iatom_0 > iatom_e
+};
+struct SplatArgs {
+    GridDev g;
+    SplatConf conf[kSplatConfs];
+    int n_conf;
+    size_t trans_stride;       // elements between the outputs of consecutive configurations
     const float* tab;          // per type 5*nR floats: R2, c0, c1, c2, c3
     const float* R_max;        // per type (float)
     int n_types;
     int nR;
     float w;                   // Vr_factor: T = exp(i*w*V)
     int wpo;                   // weak phase object: T = 1 + i*w*V
-    float2* trans;             // [n_slice][nx*ny] or null
-    float* V;                  // [n_slice][nx*ny] or null
+    float2* trans;             // [n_conf][n_slice][nx*ny] or null
+    float* V;                  // the same, or null
 };
 void launch_splat(const SplatArgs& a, int islice_0, int n_slice, cudaStream_t s);
 
