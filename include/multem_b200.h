@@ -230,6 +230,10 @@ mt_status mt_input_report(const mt_input_multislice* in, char* buf, size_t n, in
  * (mex_files_multem/ilc_multem.cu:484-518). */
 mt_status mt_multislice_run(const mt_system_conf* conf, const mt_input_multislice* in,
                             mt_output_multislice* out);
+/* The same with every image of `out` as rows [iy][ix] (transposed on the device) instead of columns
+ * [ix][iy], for callers whose arrays are row-major. No counterpart in the reference. */
+mt_status mt_multislice_run_rows(const mt_system_conf* conf, const mt_input_multislice* in,
+                                 mt_output_multislice* out);
 
 /* Run n independent simulations (different specimens, grids, simulation types), each like
  * mt_multislice_run on in[i] -> out[i]. The reference runs one input per call
@@ -270,6 +274,8 @@ mt_status mt_engine_create(const mt_system_conf* conf, const mt_input_multislice
 /* Run all phonon configurations [fp_iconf_0, pn_nconf] (Multislice::operator(),
  * src/tem_simulation.cuh:71-97) and write the output. */
 mt_status mt_engine_run(mt_engine* eng, mt_output_multislice* out);
+/* mt_engine_run with row-major images, as mt_multislice_run_rows. */
+mt_status mt_engine_run_rows(mt_engine* eng, mt_output_multislice* out);
 /* Run a subset of phonon configurations [iconf_0, iconf_e] (1-based, inclusive) and accumulate
  * their weighted detector sums into the engine's FP64 accumulators without writing output. Used to
  * shard configurations over GPUs; mt_engine_read_stem() then returns the partial sums. */

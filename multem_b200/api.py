@@ -26,12 +26,16 @@ def _conf(system_conf):
     return (system_conf or SystemConf()).to_c()
 
 
-def output_dims(params: Parameters) -> capi.MtOutputDims:
-    lib = capi.load()
-    s, keep = params.to_c()
+def _dims(lib, s) -> capi.MtOutputDims:
     d = capi.MtOutputDims()
     capi.check(lib.mt_output_query(C.byref(s), C.byref(d)))
     return d
+
+
+def output_dims(params: Parameters) -> capi.MtOutputDims:
+    lib = capi.load()
+    s, keep = params.to_c()
+    return _dims(lib, s)
 
 
 class OutputBuffers:
@@ -62,6 +66,27 @@ class OutputBuffers:
             o.m2psi_coh = _dp(self.m2psi_coh)
         self.c = o
 
+    def rows_to_dict(self):
+        """Output dict of a run that wrote row-major images (mt_*_run_rows): they are the arrays."""
+        d = self.d
+        nt, nd, nx, ny = d.n_thick, d.n_detector, d.nx, d.ny
+        res = {"dx": self.c.dx, "dy": self.c.dy, "x": self.x[:d.n_x], "y": self.y[:d.n_y], "thick": self.thick[:nt],
+               "data": []}
+        for it in range(nt):
+            e = {}
+            if self.image_tot is not None:
+                e["image_tot"] = list(self.image_tot.reshape(nt, nd, ny, nx)[it])
+            if self.image_coh is not None:
+                e["image_coh"] = list(self.image_coh.reshape(nt, nd, ny, nx)[it])
+            if self.m2psi_tot is not None:
+                e["m2psi_tot"] = self.m2psi_tot.reshape(nt, ny, nx)[it]
+            if self.psi_coh is not None:
+                e["psi_coh"] = self.psi_coh.view(np.complex128).reshape(nt, ny, nx)[it]
+            if self.m2psi_coh is not None:
+                e["m2psi_coh"] = self.m2psi_coh.reshape(nt, ny, nx)[it]
+            res["data"].append(e)
+        return res
+
     def to_dict(self):
         d = self.d
         nx, ny = d.nx, d.ny
@@ -78,8 +103,7 @@ class OutputBuffers:
             if self.m2psi_tot is not None:
                 e["m2psi_tot"] = self.m2psi_tot.reshape(d.n_thick, nx, ny)[it].T.copy()
             if self.psi_coh is not None:
-                r = self.psi_coh.reshape(d.n_thick, nx, ny, 2)[it]
-                e["psi_coh"] = (r[..., 0] + 1j * r[..., 1]).T.copy()
+                e["psi_coh"] = self.psi_coh.view(np.complex128).reshape(d.n_thick, nx, ny)[it].T.copy()
             if self.m2psi_coh is not None:
                 e["m2psi_coh"] = self.m2psi_coh.reshape(d.n_thick, nx, ny)[it].T.copy()
             res["data"].append(e)
@@ -89,12 +113,11 @@ class OutputBuffers:
 def ilc_multem(system_conf: SystemConf | None, params: Parameters) -> dict:
     """Run a full simulation (mexFunction of mex_files_multem/ilc_multem.cu:520-546)."""
     lib = capi.load()
-    d = output_dims(params)
-    buf = OutputBuffers(d)
     s, keep = params.to_c()
+    buf = OutputBuffers(_dims(lib, s))
     conf = _conf(system_conf)
-    capi.check(lib.mt_multislice_run(C.byref(conf), C.byref(s), C.byref(buf.c)))
-    return buf.to_dict()
+    capi.check(lib.mt_multislice_run_rows(C.byref(conf), C.byref(s), C.byref(buf.c)))
+    return buf.rows_to_dict()
 
 
 def ilc_multem_mat(in_path, out_path, var: str | None = None, compress: bool = False) -> None:
@@ -204,7 +227,7 @@ class Engine:
         h = C.c_void_p()
         capi.check(self.lib.mt_engine_create(C.byref(conf), C.byref(self._s), C.byref(h)))
         self.h = h
-        self.dims = output_dims(params)
+        self.dims = _dims(self.lib, self._s)
 
     def close(self):
         if self.h:
@@ -219,8 +242,8 @@ class Engine:
 
     def run(self) -> dict:
         buf = OutputBuffers(self.dims)
-        capi.check(self.lib.mt_engine_run(self.h, C.byref(buf.c)))
-        return buf.to_dict()
+        capi.check(self.lib.mt_engine_run_rows(self.h, C.byref(buf.c)))
+        return buf.rows_to_dict()
 
     def reset(self):
         capi.check(self.lib.mt_engine_reset(self.h))

@@ -101,6 +101,8 @@ SIGNATURES = {
     "mt_output_query": (c_int, [C.POINTER(MtInputMultislice), C.POINTER(MtOutputDims)]),
     "mt_multislice_run": (c_int, [C.POINTER(MtSystemConf), C.POINTER(MtInputMultislice),
                                   C.POINTER(MtOutputMultislice)]),
+    "mt_multislice_run_rows": (c_int, [C.POINTER(MtSystemConf), C.POINTER(MtInputMultislice),
+                                       C.POINTER(MtOutputMultislice)]),
     "mt_input_report": (c_int, [C.POINTER(MtInputMultislice), C.c_char_p, C.c_size_t, P_int]),
     "mt_multislice_run_batch": (c_int, [C.POINTER(MtSystemConf), c_int, C.POINTER(MtInputMultislice),
                                         C.POINTER(MtOutputMultislice), P_int]),
@@ -112,6 +114,7 @@ SIGNATURES = {
     "mt_multislice_run_mat": (c_int, [C.c_char_p, C.c_char_p, C.c_char_p, c_int]),
     "mt_engine_create": (c_int, [C.POINTER(MtSystemConf), C.POINTER(MtInputMultislice), C.POINTER(_VP)]),
     "mt_engine_run": (c_int, [_VP, C.POINTER(MtOutputMultislice)]),
+    "mt_engine_run_rows": (c_int, [_VP, C.POINTER(MtOutputMultislice)]),
     "mt_engine_run_confs": (c_int, [_VP, c_int, c_int]),
     "mt_engine_reset": (c_int, [_VP]),
     "mt_engine_read_stem": (c_int, [_VP, P_double, C.c_size_t]),

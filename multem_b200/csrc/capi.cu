@@ -106,6 +106,16 @@ mt_status mt_engine_run(mt_engine* eng, mt_output_multislice* out) {
     });
 }
 
+mt_status mt_engine_run_rows(mt_engine* eng, mt_output_multislice* out) {
+    return guarded([&] {
+        if (!eng) mtb::fail(MT_ERR_INVALID_ARG, "eng is NULL");
+        auto& e = *eng->eng;
+        e.reset();
+        e.run_confs(e.model().fp_iconf_0, e.model().pn_nconf);
+        e.write_output(out, true);
+    });
+}
+
 mt_status mt_engine_run_confs(mt_engine* eng, int iconf_0, int iconf_e) {
     return guarded([&] {
         if (!eng) mtb::fail(MT_ERR_INVALID_ARG, "eng is NULL");
@@ -219,6 +229,15 @@ mt_status mt_multislice_run(const mt_system_conf* conf, const mt_input_multislic
         mtb::Engine e(&c, in);
         e.run_confs(e.model().fp_iconf_0, e.model().pn_nconf);
         e.write_output(out);
+    });
+}
+
+mt_status mt_multislice_run_rows(const mt_system_conf* conf, const mt_input_multislice* in, mt_output_multislice* out) {
+    return guarded([&] {
+        mt_system_conf c = conf ? *conf : default_conf();
+        mtb::Engine e(&c, in);
+        e.run_confs(e.model().fp_iconf_0, e.model().pn_nconf);
+        e.write_output(out, true);
     });
 }
 

@@ -76,8 +76,7 @@ void dev_free(void* p, int dev) {
     cudaGetDevice(&cur);
     if (cur != dev) cudaSetDevice(dev);
     cudaDeviceSynchronize();
-    cudaFreeAsync(p, pool_of(dev).stream);
-    cudaStreamSynchronize(pool_of(dev).stream);
+    cudaFreeAsync(p, pool_of(dev).stream);  // ordered before every later allocation of the pool
     if (cur != dev) cudaSetDevice(cur);
 }
 
@@ -87,7 +86,6 @@ void dev_free_idle(void* p, int dev) {
     cudaGetDevice(&cur);
     if (cur != dev) cudaSetDevice(dev);
     cudaFreeAsync(p, pool_of(dev).stream);
-    cudaStreamSynchronize(pool_of(dev).stream);
     if (cur != dev) cudaSetDevice(cur);
 }
 

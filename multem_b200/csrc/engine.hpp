@@ -70,10 +70,15 @@ struct ConfData {
     DevBuf<float4> atoms;
     DevBuf<int2> ranges;
     DevBuf<float2> prop;            // per rotation, per slice then per thickness: Px[nx] then Py[ny]
+    // what ranges and prop hold, so that an equal upload is left out
+    std::vector<int2> ranges_held;
+    std::shared_ptr<const std::vector<float2>> prop_held;
     void release_idle() {
         atoms.release_idle();
         ranges.release_idle();
         prop.release_idle();
+        ranges_held.clear();
+        prop_held.reset();
     }
 };
 
@@ -99,7 +104,8 @@ class Engine {
     // graph has run, write_output reads the results.
     void prepare_run();
     void record_run();
-    void write_output(mt_output_multislice* out);
+    // rows: images as rows [iy][ix] (transposed on the device) instead of the ABI's columns [ix][iy]
+    void write_output(mt_output_multislice* out, bool rows = false);
     void read_stem(double* image_tot, size_t n);
     void cancel() { cancel_ = true; }
     void progress(int* iter, int* niter) const { *iter = iter_; *niter = niter_; }
@@ -207,13 +213,25 @@ class Engine {
     struct ConfStage {                // host staging of a configuration's device data
         std::vector<float4> at;
         std::vector<int2> rg;
-        std::vector<float2> prop;
+        std::shared_ptr<const std::vector<float2>> prop;
         size_t n_atoms = 0;
     };
     void prepare_conf_host(ConfData& cd, int iconf, ConfStage& st);
+    void prepare_batch_host(ConfData* cds, int c, int nb, ConfStage* st);
+    void pack_atoms(const AtomsF& A, std::vector<float4>& at) const;
     std::vector<float> prop_key_;     // slice thicknesses and back-propagation distances of prop_cache_
-    std::vector<float2> prop_cache_;  // propagator tables of every rotation (per slice, then per thickness)
-    void prepare_conf_device(ConfData& cd, ConfStage& st);
+    // propagator tables of every rotation (per slice, then per thickness); replaced, never changed
+    std::shared_ptr<const std::vector<float2>> prop_cache_;
+    void prepare_conf_device(ConfData& cd, ConfStage& st, cudaStream_t s);
+    // set-up of a configuration batch while the previous batch runs: its uploads' stream, and per slot
+    // group the events of its uploads and of its last run
+    cudaStream_t up_stream_ = nullptr;
+    cudaEvent_t up_done_[2] = {}, group_done_[2] = {};
+    // device to host copy of a finished result; large ones through pinned pieces by several threads
+    void copy_out(void* dst, const void* src, size_t bytes);
+    void* copy_stage_ = nullptr;
+    void copy_images(double* dst, const double* src, size_t planes, int nx, int ny, int width, bool rows);
+    DevBuf<double> d_rows_;           // transposed images
     void run_conf(ConfData& cd);
     // the splats of nb configurations (into consecutive transmission blocks) and their slice loop
     // (nb > 1: exit-wave family only, configurations with identical slicing)
@@ -243,6 +261,7 @@ class Engine {
     struct ConfGraph {
         cudaGraphExec_t exec = nullptr;
         std::vector<char> sig;  // launch-shaping data the graph was captured with
+        std::vector<char> seen;  // that of the last direct run
         int iters = 0;          // progress iterations it advances
         long long launches = 0;  // kernel launches it holds
     };
