@@ -20,6 +20,7 @@
 #include "common.hpp"
 #include "fft_core.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace mtb {
 
@@ -61,13 +62,15 @@ void encode_tile_map(CUtensorMap* map, const float2* base, int nx, int ldy, int 
 // sums the contributions of the surviving atoms in atom order in registers (deterministic, no atomics;
 // the tile size changes no sum). The epilogue writes T = exp(i*w*V) (functor::transmission_function,
 // src/cgpu_fcns.cuh:3072-3086) directly; V never goes to HBM unless asked for. Float products and sums
-// use the _rn intrinsics so they are not fused into FMAs and round like the reference's host float path.
+// use the _rn intrinsics, so that distances and knot intervals are those of the reference's host float
+// path; the cubic itself takes fused multiply-adds (one rounding a step instead of two: potentials
+// within 2e-8 of the separately rounded ones, as near to the 64-bit ones).
 //
 // Bound by instructions. A warp owns PX consecutive x of 32 consecutive y: (x - x_atom)^2 is the same
 // for its 32 lanes, so an atom whose circle does not reach a row of the warp costs that row one
 // uniform test, and (y - y_atom)^2 is computed once per atom; about 0.6 of the pixels visited lie inside
 // the circle (0.17 when each thread's pixels were spread over the whole tile). Two pixels are
-// evaluated together with packed sums and products (the same roundings), their spline interval found
+// evaluated together with packed arithmetic, their spline interval found
 // from a base-2 logarithm and two exact comparisons with one 8-byte load, the four coefficients from
 // one 16-byte load; about 25 issue cycles per warp and evaluation. Measured on one B200 per
 // configuration: Si 256^2 x 32 slices 54 -> 26 us (eight configurations in one launch), SrTiO3 512^2 x
@@ -101,6 +104,11 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
 __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
     unsigned long long d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -128,6 +136,7 @@ __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int i
     __shared__ float2 s_guess[kMaxTypes];  // log2(R2) -> interval: scale, offset
     constexpr int TX = SPLAT_WARPS * PX;
 
+    previous_done();
     const int nR = a.nR;
     float2* sm_knot = reinterpret_cast<float2*>(sm_coef + a.n_types * nR);
     for (int i = threadIdx.x; i < a.n_types * nR; i += SPLAT_THREADS) {
@@ -230,9 +239,9 @@ __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int i
                     const float d1 = __fsub_rn(R2[1], spline_interval(knot, nR, guess.x, guess.y, R2[1], i1));
                     const float4 e0 = coef[i0], e1 = coef[i1];
                     const unsigned long long d = pack2(make_float2(d0, d1));
-                    unsigned long long v = add2(mul2(pack2(make_float2(e0.w, e1.w)), d), pack2(make_float2(e0.z, e1.z)));
-                    v = add2(mul2(v, d), pack2(make_float2(e0.y, e1.y)));
-                    v = add2(mul2(v, d), pack2(make_float2(e0.x, e1.x)));
+                    unsigned long long v = fma2(pack2(make_float2(e0.w, e1.w)), d, pack2(make_float2(e0.z, e1.z)));
+                    v = fma2(v, d, pack2(make_float2(e0.y, e1.y)));
+                    v = fma2(v, d, pack2(make_float2(e0.x, e1.x)));
                     const float2 r = unpack2(mul2(occ, v));
                     V[q] = add2(V[q], pack2(make_float2(in[0] ? r.x : 0.0f, in[1] ? r.y : 0.0f)));
                 }
@@ -250,9 +259,9 @@ __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int i
                                 int i;
                                 const float dx = __fsub_rn(R2, spline_interval(knot, nR, guess.x, guess.y, R2, i));
                                 const float4 e = coef[i];
-                                float v = __fadd_rn(__fmul_rn(e.w, dx), e.z);
-                                v = __fadd_rn(__fmul_rn(v, dx), e.y);
-                                v = __fadd_rn(__fmul_rn(v, dx), e.x);
+                                float v = __fmaf_rn(e.w, dx, e.z);
+                                v = __fmaf_rn(v, dx, e.y);
+                                v = __fmaf_rn(v, dx, e.x);
                                 v = __fmul_rn(af.occ, v);
                                 float2 s = unpack2(V[p / 2]);
                                 (p % 2 ? s.y : s.x) += v;
@@ -284,6 +293,7 @@ __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int i
             a.trans[idx] = make_float2(cs, sn);
         }
     }
+    next_may_start();
 }
 
 template <int PX>
@@ -291,9 +301,8 @@ static void splat_launch(const SplatArgs& a, int islice_0, int n_slice, cudaStre
     const dim3 grid(a.g.ny / SPLAT_TY, a.g.nx / (SPLAT_WARPS * PX), n_slice * a.n_conf);
     const size_t sm = (size_t)a.n_types * a.nR * (sizeof(float4) + sizeof(float2));
     MTB_CUDA(cudaFuncSetAttribute(splat_kernel<PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    splat_kernel<PX><<<grid, SPLAT_THREADS, sm, s>>>(a, islice_0, n_slice);
+    launch_early(splat_kernel<PX>, grid, SPLAT_THREADS, sm, s, a, islice_0, n_slice);
     g_launches++;
-    MTB_CUDA(cudaGetLastError());
 }
 
 // Slices islice_0 .. islice_0 + n_slice - 1 of the n_conf configurations of `a` in one launch. Taller
@@ -390,20 +399,21 @@ void launch_cols(int nx, int flags, const ColArgs& a, int grid_ctas, cudaStream_
 __global__ void det_reduce_kernel(const double* __restrict__ partial, int nprobe, int n_tiles, int n_det,
                                   const int* __restrict__ scan_index, double w, double* __restrict__ image,
                                   int n_scan) {
+    previous_done();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nprobe * n_det) return;
     const int b = i / n_det, d = i % n_det;
     double s = 0.0;
     for (int k = 0; k < n_tiles; k++) s += partial[((size_t)b * n_tiles + k) * n_det + d];
     image[(size_t)d * n_scan + scan_index[b]] += w * s;
+    next_may_start();
 }
 
 void launch_det_reduce(const double* partial, int nprobe, int n_tiles, int n_det, const int* scan_index, double w,
                        double* image, int n_scan, cudaStream_t s) {
     const int n = nprobe * n_det;
-    det_reduce_kernel<<<(n + 127) / 128, 128, 0, s>>>(partial, nprobe, n_tiles, n_det, scan_index, w, image, n_scan);
+    launch_early(det_reduce_kernel, (n + 127) / 128, 128, 0, s, partial, nprobe, n_tiles, n_det, scan_index, w, image, n_scan);
     g_launches++;
-    MTB_CUDA(cudaGetLastError());
 }
 
 // =============================================================================================
@@ -519,6 +529,7 @@ void launch_coh_detect(const float2* coh, int n_thk, int n_scan, const ColArgs& 
 __global__ void ew_accumulate_kernel(const float2* __restrict__ psi, int nx, int ny, int ix0, int ix1, int iy0,
                                      int iy1, double w, int assign, double* __restrict__ psi_out,
                                      double* __restrict__ m2_out, int nwave) {
+    previous_done();
     const int iy = blockIdx.x * blockDim.x + threadIdx.x;
     const int ix = blockIdx.y;
     if (iy >= ny || ix >= nx) return;
@@ -545,14 +556,14 @@ __global__ void ew_accumulate_kernel(const float2* __restrict__ psi, int nx, int
         }
         m2_out[o] += acc;
     }
+    next_may_start();
 }
 
 void launch_ew_accumulate(const float2* psi, int nx, int ny, int ix0, int ix1, int iy0, int iy1, double w,
                           int assign, double* psi_out, double* m2_out, cudaStream_t s, int nwave) {
     dim3 grid((ny + 127) / 128, nx);
-    ew_accumulate_kernel<<<grid, 128, 0, s>>>(psi, nx, ny, ix0, ix1, iy0, iy1, w, assign, psi_out, m2_out, nwave);
+    launch_early(ew_accumulate_kernel, grid, 128, 0, s, psi, nx, ny, ix0, ix1, iy0, iy1, w, assign, psi_out, m2_out, nwave);
     g_launches++;
-    MTB_CUDA(cudaGetLastError());
 }
 
 // 32 x 32 tiles through shared memory, both sides coalesced.

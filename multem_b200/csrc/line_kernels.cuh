@@ -11,6 +11,7 @@
 #include "common.hpp"
 #include "fft_core.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "mbarrier.cuh"
 
 namespace mtb {
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(LineGeom<NY>::THREADS, LinePlan<NY>::B) rows_k
     const float2* twF[3] = {nullptr, nullptr, nullptr};
     setup_twiddles<NY>(smem2, twI, twF);
     float2* lines = smem2 + G::TW_I + G::TW_F;
+    previous_done();
     __syncthreads();
 
     const int li = threadIdx.x / TPL, t = threadIdx.x % TPL;
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(LineGeom<NY>::THREADS, LinePlan<NY>::B) rows_k
             for (int i = 0; i < E; i++) a.out[off + reg_pos<NY, G::R1>(i, t)] = x[i];
         }
     }
+    next_may_start();
 }
 
 template <int NY>
@@ -282,6 +285,7 @@ __global__ void __launch_bounds__(LineGeom<NX>::THREADS, LinePlan<NX>::B) cols_k
     float2* s_px = smem2 + G::TW_I + G::TW_F;
     float2* lines = s_px + (PROP ? NX : 0);
     __shared__ double s_red[NWARP][kMaxDet];
+    previous_done();
     if constexpr (PROP) {
         for (int i = threadIdx.x; i < NX; i += blockDim.x) s_px[i] = a.Px[i];
     }
@@ -347,6 +351,7 @@ __global__ void __launch_bounds__(LineGeom<NX>::THREADS, LinePlan<NX>::B) cols_k
             for (int i = 0; i < E; i++) dst[(reg_pos<NX, G::RL>(i, t) - t) * ldy] = x[i];
         }
     }
+    next_may_start();
 }
 
 template <int NX, int FLAGS>
@@ -457,11 +462,12 @@ __global__ void __launch_bounds__(GT * NG, 1) rows_pipe_kernel(RowArgs a) {
     float2* slot = slots + grp * P::SLOT;
     float2* buf = EARLY ? slots + NG * P::SLOT + grp * P::HBUF + (size_t)li * P::LBUF : slot + (size_t)li * G::LS;
     if (threadIdx.x == 0) {
-        s_skip = err_set(a.err);  // an earlier pass timed out: the CTA returns (one decision for all)
         for (int i = 0; i < NG; i++) mbar_init(&full[i], 1);
         mbar_init(&tbar, 1);
         mbar_fence_init();
     }
+    previous_done();
+    if (threadIdx.x == 0) s_skip = err_set(a.err);  // an earlier pass timed out: the CTA returns (one decision for all)
     __syncthreads();
     if (s_skip) return;
 
@@ -576,6 +582,7 @@ __global__ void __launch_bounds__(GT * NG, 1) rows_pipe_kernel(RowArgs a) {
     // copies this warp issued and nobody saw land (only after an error): wait them out
     if (gtid == 0 && last_k >= 0) mbar_drain(&full[grp], (unsigned)(last_k / NG) & 1u);
     if (threadIdx.x == 0 && last_tph >= 0) mbar_drain(&tbar, (unsigned)last_tph);
+    next_may_start();
 }
 
 // Row-pass pipeline shapes per line length: threads per group, groups, pipeline mode. Shape 0 is
@@ -670,14 +677,15 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     float2* land = land0 + grp * P::LAND;
     float2* buf = EARLY ? land0 + NG * P::LAND + grp * P::HBUF + (size_t)c * P::LSH : land + (size_t)c * P::LSH;
     (void)HALF;
-    if constexpr (PROP) {
-        for (int i = threadIdx.x; i < NX; i += blockDim.x) s_px[i] = a.Px[i];
-    }
     if (threadIdx.x == 0) {
-        s_skip = err_set(a.err);  // an earlier pass timed out: the CTA returns (one decision for all)
         for (int i = 0; i < NG; i++) mbar_init(&full[i], 1);
         mbar_fence_init();
     }
+    previous_done();
+    if constexpr (PROP) {
+        for (int i = threadIdx.x; i < NX; i += blockDim.x) s_px[i] = a.Px[i];
+    }
+    if (threadIdx.x == 0) s_skip = err_set(a.err);  // an earlier pass timed out: the CTA returns (one decision for all)
     __syncthreads();
     if (s_skip) return;
 
@@ -772,6 +780,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     }
     // a tile this thread issued and nobody saw land (only after an error): wait it out
     if (gtid == 0 && last_k >= 0) mbar_drain(&full[grp], (unsigned)(last_k / NG) & 1u);
+    next_may_start();
 }
 
 // Tensor map for cols_pipe_kernel over a probe batch at `base` (cuTensorMapEncodeTiled through
@@ -810,9 +819,8 @@ static bool rows_pipe_try(const RowArgs& a, int grid_ctas, cudaStream_t s) {
         const int units = (a.nx / RP::LPC) * a.nprobe / S::NG;
         int grid = grid_ctas > 0 ? grid_ctas : cap;
         if (grid > units) grid = units;
-        kern<<<grid, S::GT * S::NG, RP::SMEM, s>>>(a);
+        launch_early(kern, grid, S::GT * S::NG, RP::SMEM, s, a);
         note_launch();
-        MTB_CUDA(cudaGetLastError());
         return true;
     } else {
         (void)a, (void)grid_ctas, (void)s;
@@ -838,9 +846,8 @@ static void rows_launch(const RowArgs& a, int grid_ctas, cudaStream_t s) {
     const int items = (a.nx / G::LPC) * a.nprobe;
     int grid = grid_ctas > 0 ? grid_ctas : cap;
     if (grid > items) grid = items;
-    rows_kernel<NY, MODE><<<grid, G::THREADS, sm, s>>>(a);
+    launch_early(rows_kernel<NY, MODE>, grid, G::THREADS, sm, s, a);
     note_launch();
-    MTB_CUDA(cudaGetLastError());
 }
 
 template <int NY>
@@ -867,9 +874,8 @@ static bool cols_pipe_try(const ColArgs& a, int grid_ctas, cudaStream_t s) {
         if (grid > items) grid = items;
         CUtensorMap map;
         encode_tile_map(&map, a.in, NX, a.ny, a.nprobe, CP::W, CP::BOXR);
-        kern<<<grid, S::GT * S::NG, CP::SMEM, s>>>(a, map);
+        launch_early(kern, grid, S::GT * S::NG, CP::SMEM, s, a, map);
         note_launch();
-        MTB_CUDA(cudaGetLastError());
         return true;
     } else {
         (void)a, (void)grid_ctas, (void)s;
@@ -892,9 +898,8 @@ static void cols_launch_ld(const ColArgs& a, int grid_ctas, cudaStream_t s) {
     const int items = (a.ny / G::LPC) * a.nprobe;
     int grid = grid_ctas > 0 ? grid_ctas : cap;
     if (grid > items) grid = items;
-    cols_kernel<NX, FLAGS, LDY><<<grid, G::THREADS, sm, s>>>(a);
+    launch_early(cols_kernel<NX, FLAGS, LDY>, grid, G::THREADS, sm, s, a);
     note_launch();
-    MTB_CUDA(cudaGetLastError());
 }
 
 template <int NX, int FLAGS>
