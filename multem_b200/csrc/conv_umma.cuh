@@ -24,6 +24,7 @@
 
 #include <cstdint>
 
+#include "launch.cuh"
 #include "mbarrier.cuh"
 
 namespace mtb {
@@ -381,6 +382,10 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
         s_off[s] = pixel_offset(a.im, a.Cin, b0, r0, (ky - 1) * Wp - 1 + j);
     }
     tc_fence_before();
+    __syncthreads();
+    // only now, so that no CTA of a later kernel can hold tensor memory that one of this kernel waits for
+    next_may_start();
+    previous_done();
     const __nv_bfloat16* in = a.in + (size_t)b0 * a.Cin * hw;
     const __nv_bfloat16* mask = a.mask ? a.mask + (size_t)b0 * a.Cin * hw : nullptr;
 
@@ -407,7 +412,6 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
                 for (int t = 0; t < 9; t++) wt[((8 - t) * (BN / 8) + p) * kw + k] = v[t];
             }
         }
-        if (kb == 0) __syncthreads();  // the offsets
         gather({in, mask, hw, a.Cin}, s_off, (kb0 + kb) * kw, nplane, npix, reinterpret_cast<uint4*>(st), [](uint4) {});
         fence_proxy_async();
         __syncthreads();
@@ -585,6 +589,8 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = s_tmem;
+    next_may_start();  // after the allocation, as in conv_kernel
+    previous_done();
 
     const int blk0 = blockIdx.x * a.blk_per_split;
     const int nb = a.nblk - blk0 < a.blk_per_split ? a.nblk - blk0 : a.blk_per_split;
@@ -720,6 +726,8 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
 __global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, int splits, int itiles, int NI,
                                                              float* __restrict__ dw, float* __restrict__ db) {
     __shared__ float s[8][3][32];
+    next_may_start();
+    previous_done();
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int o = blockIdx.x * 32 + lane, i = blockIdx.y, ky = blockIdx.z, C32 = gridDim.x * 32;
     const bool bias = i == a.Cin;

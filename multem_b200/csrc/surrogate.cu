@@ -39,6 +39,8 @@ __global__ void surrogate_loss_kernel(const float* __restrict__ head, const __nv
                                       const float* __restrict__ t, const float* __restrict__ scale,
                                       __nv_bfloat16* __restrict__ dhead, float* __restrict__ terms, int B, int HW,
                                       float lambda) {
+    mtb::next_may_start();
+    mtb::previous_done();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= B * HW) return;
     const int b = p / HW, q = p % HW;
@@ -57,6 +59,8 @@ __global__ void surrogate_loss_kernel(const float* __restrict__ head, const __nv
 __global__ void adam_kernel(float* __restrict__ wm, __nv_bfloat16* __restrict__ wb, const float* __restrict__ g,
                             float* __restrict__ m, float* __restrict__ v, int n, float lr, float b1, float b2, float eps,
                             float c1, float c2) {
+    mtb::next_may_start();
+    mtb::previous_done();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -73,6 +77,8 @@ __global__ void adam_kernel(float* __restrict__ wm, __nv_bfloat16* __restrict__ 
 // the gradient of nearest-neighbour upsampling with scale 1.
 __global__ void pool2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int planes, int H,
                              int W, float scale) {
+    mtb::next_may_start();
+    mtb::previous_done();
     const int Ho = H / 2, Wo = W / 2;
     const size_t n = (size_t)planes * Ho * Wo;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -88,6 +94,8 @@ __global__ void pool2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16
 // scale 1, the gradient of average pooling with scale 1/4.
 __global__ void upsample2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int planes,
                                  int H, int W, float scale) {
+    mtb::next_may_start();
+    mtb::previous_done();
     const int Ho = 2 * H, Wo = 2 * W;
     const size_t n = (size_t)planes * Ho * Wo;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -99,6 +107,8 @@ __global__ void upsample2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bflo
 
 __global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                            __nv_bfloat16* __restrict__ out, size_t n) {
+    mtb::next_may_start();
+    mtb::previous_done();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         out[k] = __float2bfloat16_rn(bf(a[k]) + bf(b[k]));
 }
@@ -177,12 +187,14 @@ void conv_launch(const mtb::conv::ConvArgs& a, cudaStream_t st) {
     cfg.blockDim = dim3(mtb::conv::THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = (unsigned)a.ksplit;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = (unsigned)a.ksplit;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as mtb::launch_early
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
     MTB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
 }
 
@@ -228,11 +240,9 @@ void wgrad_launch(mtb::conv::WgradArgs a, float* dw, float* db, cudaStream_t st)
     auto kern = mtb::conv::wgrad_kernel<NI>;
     const size_t smem = T::smem(a.im.W);
     MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<dim3((unsigned)splits, (unsigned)itiles, (unsigned)otiles), mtb::conv::THREADS, smem, st>>>(a);
-    MTB_CUDA(cudaGetLastError());
-    mtb::conv::wgrad_finalize_kernel<<<dim3((unsigned)otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st>>>(a, splits, itiles, NI,
-                                                                                                   dw, db);
-    MTB_CUDA(cudaGetLastError());
+    mtb::launch_early(kern, dim3((unsigned)splits, (unsigned)itiles, (unsigned)otiles), mtb::conv::THREADS, smem, st, a);
+    mtb::launch_early(mtb::conv::wgrad_finalize_kernel, dim3((unsigned)otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st, a, splits,
+                      itiles, NI, dw, db);
 }
 
 }  // namespace
@@ -313,9 +323,8 @@ mt_status mt_sg_loss(const float* head, const void* x, const float* target, cons
         check_shape(B, 1, 2, H, W);
         if (!head || !x || !target || !dhead || !terms) mtb::fail(MT_ERR_INVALID_ARG, "NULL tensor");
         const int n = B * H * W;
-        surrogate_loss_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-            head, (const __nv_bfloat16*)x, target, scale, (__nv_bfloat16*)dhead, terms, B, H * W, lambda);
-        MTB_CUDA(cudaGetLastError());
+        mtb::launch_early(surrogate_loss_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, head, (const __nv_bfloat16*)x,
+                          target, scale, (__nv_bfloat16*)dhead, terms, B, H * W, lambda);
     });
 }
 
@@ -324,9 +333,8 @@ mt_status mt_sg_adam(float* w, void* w_bf16, const float* g, float* m, float* v,
     return run([&] {
         if (n <= 0 || step <= 0) mtb::fail(MT_ERR_INVALID_ARG, "bad Adam arguments");
         const float c1 = 1.0f - std::pow(b1, (float)step), c2 = 1.0f - std::pow(b2, (float)step);
-        adam_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(w, (__nv_bfloat16*)w_bf16, g, m, v, n, lr, b1, b2,
-                                                                        eps, c1, c2);
-        MTB_CUDA(cudaGetLastError());
+        mtb::launch_early(adam_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, w, (__nv_bfloat16*)w_bf16, g, m, v, n,
+                          lr, b1, b2, eps, c1, c2);
     });
 }
 
@@ -336,9 +344,8 @@ mt_status mt_sg_pool2(const void* in, void* out, int B, int C, int H, int W, flo
         if (H % 2 || W % 2) mtb::fail(MT_ERR_INVALID_ARG, "pooling needs even H and W");
         if (!in || !out) mtb::fail(MT_ERR_INVALID_ARG, "NULL tensor");
         const size_t n = (size_t)B * C * (H / 2) * (W / 2);
-        pool2_kernel<<<elem_grid(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, B * C,
-                                                                     H, W, scale);
-        MTB_CUDA(cudaGetLastError());
+        mtb::launch_early(pool2_kernel, elem_grid(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+                          (__nv_bfloat16*)out, B * C, H, W, scale);
     });
 }
 
@@ -347,9 +354,8 @@ mt_status mt_sg_upsample2(const void* in, void* out, int B, int C, int H, int W,
         check_shape(B, C, 1, 2 * H, 2 * W);
         if (!in || !out) mtb::fail(MT_ERR_INVALID_ARG, "NULL tensor");
         const size_t n = (size_t)B * C * (2 * H) * (2 * W);
-        upsample2_kernel<<<elem_grid(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out,
-                                                                         B * C, H, W, scale);
-        MTB_CUDA(cudaGetLastError());
+        mtb::launch_early(upsample2_kernel, elem_grid(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+                          (__nv_bfloat16*)out, B * C, H, W, scale);
     });
 }
 
@@ -357,9 +363,8 @@ mt_status mt_sg_add(const void* a, const void* b, void* out, long long n, void* 
     return run([&] {
         if (n < 0 || (n > 0 && (!a || !b || !out))) mtb::fail(MT_ERR_INVALID_ARG, "bad add arguments");
         if (n == 0) return;
-        add_kernel<<<elem_grid((size_t)n), 256, 0, (cudaStream_t)stream>>>(
-            (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, (size_t)n);
-        MTB_CUDA(cudaGetLastError());
+        mtb::launch_early(add_kernel, elem_grid((size_t)n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)a,
+                          (const __nv_bfloat16*)b, (__nv_bfloat16*)out, (size_t)n);
     });
 }
 
