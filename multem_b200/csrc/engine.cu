@@ -1044,10 +1044,10 @@ void Engine::run_conf_batch(ConfData* const* cds, int nb) {
 
 // Autotuner of the line passes. For each (nx, ny, allocated probes per launch) the process times,
 // once, on this engine's probe buffer, transmission function and propagator (one warm-up and three
-// timed launches each): the row pass and the column pass of the slice step in each variant (per-
-// thread loads; bulk-copy fed; bulk-copy fed in the alternative pipeline shapes RowPipeShape<N, 1|2>
-// and ColPipeShape<N, 1|2>: narrower groups, and early issue with full exchange buffers in as many
-// groups as shared memory holds), keeping the fastest of each; then, for STEM batches of at least 16
+// timed launches each, twice over): the row pass and the column pass of the slice step in each variant
+// (per-thread loads; bulk-copy fed; bulk-copy fed in the alternative pipeline shapes 1 and 2 of
+// RowPipeShape and ColPipeShape, where a length has them), keeping the fastest of each; then, for STEM
+// batches of at least 16
 // probes, the chosen step at the full and at half the batch, keeping the batch with the lower
 // time per probe. Every variant computes the same transforms with the same rounding, so the
 // choice changes only the speed (the FP64 detector partials of other tile widths are added in
@@ -1110,10 +1110,14 @@ Engine::Tuning Engine::tune_passes(int nprobe, ConfData& cd) {
     };
     constexpr int NV = 4;
     float tr[NV], tc[NV];
-    for (int v = 0; v < NV; v++) {
-        tr[v] = rows_t(v, nprobe);
-        tc[v] = cols_t(v, nprobe);
-    }
+    // two rounds over the variants, each keeping its faster one: clocks and power settle during the
+    // first, and one disturbed measurement decides nothing
+    for (int round = 0; round < 2; round++)
+        for (int v = 0; v < NV; v++) {
+            const float r = rows_t(v, nprobe), c = cols_t(v, nprobe);
+            tr[v] = round ? std::min(tr[v], r) : r;
+            tc[v] = round ? std::min(tc[v], c) : c;
+        }
     int vr = 0, vc = 0;
     for (int v = 1; v < NV; v++) {
         if (tr[v] < tr[vr]) vr = v;

@@ -554,6 +554,50 @@ __device__ __forceinline__ void stage_exchange_half(float2* x, float2* buf, int 
     });
 }
 
+// Exchange after stage S that also changes the owner: this thread writes as thread tw of line buffer bw and
+// reads as thread tr of line buffer br. Lines are written by threads of one warp (synchronised here)
+// and read by any of the group, whose barrier is `sync`; earlier readers of the buffers must have passed
+// a barrier of the group. HALF takes the two-round half-line exchange.
+template <int N, bool REV, int S, bool HALF, class Sync>
+__device__ __forceinline__ void stage_exchange_owner(float2* x, float2* bw, int tw, const float2* br, int tr, Sync sync) {
+    __syncwarp();
+    if constexpr (HALF) {
+        using H = HalfExchange<N, REV>;
+        using M = HalfExchangeMap<N, REV>;
+        static_assert(M::LINEAR && S == 0, "half-line exchange of a two-stage plan");
+        static_for<0, 2>([&](auto hc) {
+            constexpr int h = decltype(hc)::value;
+            if constexpr (h == 1) sync();
+            static_for<0, H::E>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                if constexpr (((M::wcpos(i) >> H::B) & 1) == h) bw[tw * M::SW + M::wpos(0, i)] = x[i];
+            });
+            sync();
+            static_for<0, H::E>([&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                if constexpr (((M::rcpos(i) >> H::B) & 1) == h) x[i] = br[tr * M::SR + M::rpos(0, i)];
+            });
+        });
+    } else {
+        using M = ExchangeMap<N, REV, S>;
+        static_for<0, M::E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            if constexpr (M::LINEAR) {
+                bw[tw * M::SW + M::wpos(0, i)] = x[i];
+            } else {
+                const int j = tw + M::TPL * (i / M::R);
+                bw[pad_idx<M::R>((j / M::NSV) * M::NSV * M::R + (j % M::NSV) + (i % M::R) * M::NSV)] = x[i];
+            }
+        });
+        sync();
+        static_for<0, M::E>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            if constexpr (M::LINEAR) x[i] = br[tr * M::SR + M::rpos(0, i)];
+            else x[i] = br[pad_idx<M::R>(tr + M::TPL * (i / M::R2) + (i % M::R2) * (N / M::R2))];
+        });
+    }
+}
+
 // Two-stage transform with the half-line exchange (see line_fft below).
 template <int N, bool REV, int DIR, class Sync>
 __device__ __forceinline__ void line_fft_half(float2* x, float2* buf, const float2* const* tw, int t, Sync sync) {
@@ -572,6 +616,20 @@ __device__ __forceinline__ void line_fft(float2* x, float2* buf, const float2* c
         constexpr int s = decltype(sc)::value;
         stage_compute<N, REV, s, DIR>(x, t, tw[s]);
         if constexpr (s + 1 < NSTAGE) stage_exchange<N, REV, s>(x, buf, t, sync);
+    });
+}
+
+// line_fft whose last exchange changes the owner (stage_exchange_owner): the stages before it run as thread
+// tw of the line in bw (exchanges within a warp), the last one as thread tr of the line in br.
+template <int N, bool REV, int DIR, bool HALF, class Sync>
+__device__ __forceinline__ void line_fft_owner(float2* x, float2* bw, int tw, const float2* br, int tr,
+                                               const float2* const* tab, Sync sync) {
+    constexpr int NSTAGE = LinePlan<N>::NS;
+    static_for<0, NSTAGE>([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        stage_compute<N, REV, s, DIR>(x, s + 1 < NSTAGE ? tw : tr, tab[s]);
+        if constexpr (s + 2 < NSTAGE) stage_exchange<N, REV, s>(x, bw, tw, [] { __syncwarp(); });
+        else if constexpr (s + 1 < NSTAGE) stage_exchange_owner<N, REV, s, HALF>(x, bw, tw, br, tr, sync);
     });
 }
 

@@ -585,14 +585,14 @@ __global__ void __launch_bounds__(GT * NG, 1) rows_pipe_kernel(RowArgs a) {
     next_may_start();
 }
 
-// Row-pass pipeline shapes per line length: threads per group, groups, pipeline mode. Shape 0 is
-// the default of every row pass (early issue with the half-line exchange where the plan has one,
-// else late issue); shape 1, one warp per group (so a group synchronises with __syncwarp only) and
-// 16 groups, and shape 2, early issue with full exchange buffers in as many groups (8, 4 or 2) as
-// shared memory holds, are the alternatives the autotuner may pick for the slice step.
+// Row-pass pipeline shapes per line length: threads per group, groups, pipeline mode. Shape 0 is the
+// default of every row pass (early issue with the half-line exchange where the plan has one, else late
+// issue); shape 2, early issue with full exchange buffers in as many groups (8, 4 or 2) as shared
+// memory holds, is the alternative that the autotuner may pick for the slice step where it has been the
+// faster: 256 (61 -> 55 us per 256 waves) and 2048 (360 -> 356 us per 16).
 template <int NY, int V = 0>
 struct RowPipeShape {
-    static constexpr int GT = V == 0 ? 64 : 32, NG = V == 0 ? 8 : 16;
+    static constexpr int GT = 64, NG = 8;
     static constexpr int PM = (HalfExchange<NY, false>::OK && HalfExchange<NY, true>::OK) ? 1 : 0;
 };
 template <int NY>
@@ -613,7 +613,7 @@ struct RowPipeShape<NY, 2> {
 //   PM 0: (lengths without a half-line exchange, 1024) the slot doubles as the full exchange
 //         buffer and the next tile is issued once the group's last exchange read is done; the other
 //         groups keep the copy engine busy meanwhile.
-template <int NX, int GT, int NG, int PM = (HalfExchange<NX, false>::OK && HalfExchange<NX, true>::OK) ? 1 : 0>
+template <int NX, int GT, int NG, int PM = (HalfExchange<NX, false>::OK && HalfExchange<NX, true>::OK) ? 1 : 0, bool OWN = false>
 struct ColPipe {
     using G = LineGeom<NX>;
     static constexpr int PM_V = PM;
@@ -623,9 +623,10 @@ struct ColPipe {
     static constexpr size_t TW = (size_t)G::TW_I + G::TW_F;
     static constexpr size_t LAND0 = (size_t)W * NX;
     static constexpr size_t LAND1 = EARLY ? LAND0 : ((size_t)W * LSH > LAND0 ? (size_t)W * LSH : LAND0);
-    static constexpr size_t LAND = (LAND1 + 15) / 16 * 16;  // slots on 128-byte boundaries (bulk-copy targets)
+    static constexpr size_t ALIGN = OWN ? 128 : 16;  // slots on 128-byte boundaries, swizzled ones (OWN) on 1024-byte ones
+    static constexpr size_t LAND = (LAND1 + ALIGN - 1) / ALIGN * ALIGN;
     static constexpr size_t HBUF = EARLY ? (size_t)W * LSH : 0;
-    static constexpr size_t SMEM = sizeof(float2) * (TW + NX + NG * LAND + NG * HBUF);
+    static constexpr size_t SMEM = sizeof(float2) * (TW + NX + NG * LAND + NG * HBUF + (OWN ? ALIGN : 0));
     // rows per bulk-copy box: the boxes must tile the NX rows exactly (a box reaching past NX would
     // write past the slot and count bytes the barrier does not expect)
     static constexpr int BOXR = (NX <= 256) ? NX : (NX % 256 == 0) ? 256 : (NX % 128 == 0) ? 128 : 0;
@@ -636,25 +637,53 @@ struct ColPipe {
                                (HBUF % 2 == 0) && SMEM <= kPipeSmemMax && (GT == 32 || NG <= 14);
 };
 
-// Column-pass pipeline shapes: 2 groups of 256 threads (default), and the alternatives the
-// autotuner may pick for the slice step: 4 groups of 128 threads (narrower tiles), and groups of
-// 128 threads in early-issue mode with full exchange buffers, as many (4, 3 or 2) as shared memory
-// holds.
+// Column-pass pipeline shapes: 2 groups of 256 threads (default), and the alternatives the autotuner
+// may pick for the slice step: 1, whole-line ownership (OWN below) where it is the fastest (512: the
+// default's groups; 256: six groups of 128 threads on narrower tiles), and 2, groups of 128 threads in
+// early-issue mode with full exchange buffers, as many (4, 3 or 2) as shared memory holds, at 384 and
+// 1024. One B200, us per launch (default / 1 / 2): 256^2 x 256 waves 74 / 59 / 61, 384^2 x 196 153 / - / 130,
+// 512^2 x 256 227 / 215 / 219, 1024^2 x 64 261 / - / 253, 2048^2 x 16 348 / - / 413. Ownership loses where the exchange buffer is the landing buffer itself (default 384 and 1024: 153 -> 164, 261 ->
+// 271) or few warps are left to a group (shape 2 of 384: 130 -> 145).
 template <int NX, int V = 0>
 struct ColPipeShape {
-    static constexpr int GT = V == 0 ? 256 : 128, NG = V == 0 ? 2 : 4;
+    static constexpr int GT = 256, NG = 2;
     static constexpr int PM = (HalfExchange<NX, false>::OK && HalfExchange<NX, true>::OK) ? 1 : 0;
+    static constexpr bool OWN = V == 1 && NX == 512;
+};
+template <>
+struct ColPipeShape<256, 1> {
+    static constexpr int GT = 128, NG = 6, PM = 2;
+    static constexpr bool OWN = true;
 };
 template <int NX>
 struct ColPipeShape<NX, 2> {
     static constexpr int GT = 128, PM = 2;
     static constexpr int NG = ColPipe<NX, 128, 4, 2>::OK ? 4 : ColPipe<NX, 128, 3, 2>::OK ? 3 : 2;
+    static constexpr bool OWN = false;
 };
 
-template <int NX, int FLAGS, int LDY, int GT, int NG, int PM>
+// Whole-line ownership (OWN): until the inverse transform's last exchange a thread belongs to the line that
+// its warp (or half of it) owns, so the forward transform and its exchanges synchronise one warp only; that
+// last exchange hands the points to the threads that store them in rows of W columns. Of the nine (full
+// exchange buffers: five) barriers of a group per tile four (two) are left, and the warps of a group
+// drift apart between them instead of loading and computing in step. A half-warp then reads 16 rows of one
+// column from the landing buffer, which the copy's 128- (64-) byte swizzle spreads over the banks (two
+// rows to a bank).
+template <int NX, int GT, int PM>
+struct ColOwn {
+    static constexpr int W = GT / LineGeom<NX>::TPL;
+    static constexpr int ROW = W * (int)sizeof(float2);  // bytes of a tile row: the swizzle's span
+    static constexpr bool OK = (LineGeom<NX>::TPL == 16 || LineGeom<NX>::TPL == 32) && (ROW == 128 || ROW == 64) &&
+                               (NX / LineGeom<NX>::R1) % 8 == 0 &&
+                               (PM != 1 || (HalfExchangeMap<NX, false>::LINEAR && HalfExchangeMap<NX, true>::LINEAR));
+    // 16-byte piece of a row that the swizzle moves column c of row t (mod 8 rows) to
+    static __device__ __forceinline__ int piece(int c, int t) { return (c >> 1) ^ (ROW == 128 ? t & 7 : (t >> 1) & 3); }
+};
+
+template <int NX, int FLAGS, int LDY, int GT, int NG, int PM, bool OWN>
 __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const __grid_constant__ CUtensorMap map) {
     using G = LineGeom<NX>;
-    using P = ColPipe<NX, GT, NG, PM>;
+    using P = ColPipe<NX, GT, NG, PM, OWN>;
     constexpr bool EARLY = PM != 0, HALF = PM == 1;
     constexpr int E = G::E, W = P::W, NWARP = GT / 32;
     constexpr bool PROP = FLAGS & COL_PROP, DET = FLAGS & COL_DETECT;
@@ -672,8 +701,11 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     setup_twiddles<NX>(sm, twP, twR);
     float2* s_px = sm + P::TW;
     float2* land0 = s_px + NX;  // NG landing buffers, [row][W] each
+    if constexpr (OWN) land0 += ((1024 - (smem_u32(land0) & 1023)) & 1023) / sizeof(float2);  // the swizzle's period
     const int grp = threadIdx.x / GT, gtid = threadIdx.x % GT;
-    const int c = gtid % W, t = gtid / W;
+    const int cs = gtid % W, ts = gtid / W;  // column and line thread that this thread stores
+    const int c = OWN ? gtid / G::TPL : cs, t = OWN ? gtid % G::TPL : ts;  // ... and transforms
+    static_assert(!OWN || (ColOwn<NX, GT, PM>::OK && INV), "whole-line ownership needs a swizzled tile and an inverse");
     float2* land = land0 + grp * P::LAND;
     float2* buf = EARLY ? land0 + NG * P::LAND + grp * P::HBUF + (size_t)c * P::LSH : land + (size_t)c * P::LSH;
     (void)HALF;
@@ -711,23 +743,27 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     if (gtid == 0 && grp < K) issue(grp);
 
     using GSync = typename std::conditional<(GT == 32), WarpSync, GroupSync<GT>>::type;
+    using FSync = typename std::conditional<OWN, WarpSync, GSync>::type;
     const GSync gsync{grp};
+    const FSync fsync{grp};
     for (int k = grp; k < K; k += NG) {
         const int item = blockIdx.x + k * gridDim.x;
         const int b = item / tiles, ct = item % tiles;
         const int iy = ct * W + c;
-        const size_t off = (size_t)b * pstride + iy + (size_t)t * ldy;
-        float2* dst = a.out + off;
+        float2* dst = a.out + (size_t)b * pstride + (ct * W + cs) + (size_t)ts * ldy;
         mbar_wait(&full[grp], (unsigned)(k / NG) & 1u, a.err, a.wait_ns);
         float2 x[E];
 #pragma unroll
-        for (int i = 0; i < E; i++) x[i] = land[(size_t)reg_pos<NX, G::R1>(i, t) * W + c];
+        for (int i = 0; i < E; i++) {
+            const int at = OWN ? 2 * ColOwn<NX, GT, PM>::piece(c, t) + (c & 1) : c;
+            x[i] = land[(size_t)reg_pos<NX, G::R1>(i, t) * W + at];
+        }
         gsync();  // the whole group has read its landing buffer
         if constexpr (EARLY) {
             if (gtid == 0 && k + NG < K) issue(k + NG);
         }
-        if constexpr (HALF) line_fft_half<NX, false, -1>(x, buf, twP, t, gsync);
-        else line_fft<NX, false, -1>(x, buf, twP, t, gsync);
+        if constexpr (HALF) line_fft_half<NX, false, -1>(x, buf, twP, t, fsync);
+        else line_fft<NX, false, -1>(x, buf, twP, t, fsync);
         if constexpr (PROP) {
             const float2 py = a.Py[iy];
 #pragma unroll
@@ -756,7 +792,13 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
             gsync();
         }
         if constexpr (INV) {
-            if constexpr (HALF) {
+            if constexpr (OWN) {
+                line_fft_owner<NX, true, +1, HALF>(x, buf, t, buf + (ptrdiff_t)(cs - c) * P::LSH, ts, twR, gsync);
+                if constexpr (!EARLY) {
+                    gsync();  // every exchange read of the slot is done
+                    if (gtid == 0 && k + NG < K) issue(k + NG);
+                }
+            } else if constexpr (HALF) {
                 line_fft_half<NX, true, +1>(x, buf, twR, t, gsync);
             } else {
                 line_fft<NX, true, +1>(x, buf, twR, t, gsync);
@@ -766,7 +808,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
                 }
             }
 #pragma unroll
-            for (int i = 0; i < E; i++) dst[(reg_pos<NX, G::R1>(i, t) - t) * ldy] = x[i];
+            for (int i = 0; i < E; i++) dst[(reg_pos<NX, G::R1>(i, ts) - ts) * ldy] = x[i];
             continue;
         }
         if constexpr (!EARLY) {
@@ -775,7 +817,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
         }
         if constexpr (STORE) {
 #pragma unroll
-            for (int i = 0; i < E; i++) dst[(reg_pos<NX, G::RL>(i, t) - t) * ldy] = x[i];
+            for (int i = 0; i < E; i++) dst[(reg_pos<NX, G::RL>(i, ts) - ts) * ldy] = x[i];
         }
     }
     // a tile this thread issued and nobody saw land (only after an error): wait it out
@@ -785,7 +827,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
 
 // Tensor map for cols_pipe_kernel over a probe batch at `base` (cuTensorMapEncodeTiled through
 // the runtime's driver entry point, so the library needs no link to the driver library).
-void encode_tile_map(CUtensorMap* map, const float2* base, int nx, int ldy, int nprobe, int w, int boxr);
+void encode_tile_map(CUtensorMap* map, const float2* base, int nx, int ldy, int nprobe, int w, int boxr, bool swizzle);
 
 // ---------------------------------------------------------------------------------------------
 // launch helpers (the per-kernel occupancy caps are function-local statics, initialised once and
@@ -830,15 +872,13 @@ static bool rows_pipe_try(const RowArgs& a, int grid_ctas, cudaStream_t s) {
 
 // The bulk-copy-fed kernels run where their shared memory fits and the pass loads its input;
 // they need the error flag of their bounded waits (a.err), and without it the per-thread-load
-// kernels run. The slice step may use an alternative pipeline shape (a.shape 1 or 2).
+// kernels run. The slice step may use an alternative pipeline shape (a.shape).
 template <int NY, int MODE>
 static void rows_launch(const RowArgs& a, int grid_ctas, cudaStream_t s) {
     using G = LineGeom<NY>;
     if (a.err) {
-        if constexpr (MODE == ROW_STEP) {
-            if (a.shape == 1 && rows_pipe_try<NY, MODE, 1>(a, grid_ctas, s)) return;
+        if constexpr (MODE == ROW_STEP && (NY == 256 || NY == 2048))
             if (a.shape == 2 && rows_pipe_try<NY, MODE, 2>(a, grid_ctas, s)) return;
-        }
         if (rows_pipe_try<NY, MODE, 0>(a, grid_ctas, s)) return;
     }
     const size_t sm = rows_smem<NY>();
@@ -865,15 +905,15 @@ void rows_dispatch_mode(RowMode mode, const RowArgs& a, int grid_ctas, cudaStrea
 template <int NX, int FLAGS, int LDY, int V>
 static bool cols_pipe_try(const ColArgs& a, int grid_ctas, cudaStream_t s) {
     using S = ColPipeShape<NX, V>;
-    using CP = ColPipe<NX, S::GT, S::NG, S::PM>;
+    using CP = ColPipe<NX, S::GT, S::NG, S::PM, S::OWN>;
     if constexpr (CP::OK && (FLAGS & COL_LOAD)) {
-        auto kern = cols_pipe_kernel<NX, FLAGS, LDY, S::GT, S::NG, S::PM>;
+        auto kern = cols_pipe_kernel<NX, FLAGS, LDY, S::GT, S::NG, S::PM, S::OWN>;
         static const int cap = max_ctas(kern, S::GT * S::NG, CP::SMEM);
         const int items = (a.ny / CP::W) * a.nprobe;
         int grid = grid_ctas > 0 ? grid_ctas : cap;
         if (grid > items) grid = items;
         CUtensorMap map;
-        encode_tile_map(&map, a.in, NX, a.ny, a.nprobe, CP::W, CP::BOXR);
+        encode_tile_map(&map, a.in, NX, a.ny, a.nprobe, CP::W, CP::BOXR, S::OWN);
         launch_early(kern, grid, S::GT * S::NG, CP::SMEM, s, a, map);
         note_launch();
         return true;
@@ -888,8 +928,10 @@ static void cols_launch_ld(const ColArgs& a, int grid_ctas, cudaStream_t s) {
     using G = LineGeom<NX>;
     if (a.err) {
         if constexpr (FLAGS == (COL_LOAD | COL_PROP | COL_INVERSE | COL_STORE)) {
-            if (a.shape == 1 && cols_pipe_try<NX, FLAGS, LDY, 1>(a, grid_ctas, s)) return;
-            if (a.shape == 2 && cols_pipe_try<NX, FLAGS, LDY, 2>(a, grid_ctas, s)) return;
+            if constexpr (ColPipeShape<NX, 1>::OWN)
+                if (a.shape == 1 && cols_pipe_try<NX, FLAGS, LDY, 1>(a, grid_ctas, s)) return;
+            if constexpr (NX == 384 || NX == 1024)
+                if (a.shape == 2 && cols_pipe_try<NX, FLAGS, LDY, 2>(a, grid_ctas, s)) return;
         }
         if (cols_pipe_try<NX, FLAGS, LDY, 0>(a, grid_ctas, s)) return;
     }

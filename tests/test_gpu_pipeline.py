@@ -63,9 +63,9 @@ def test_exit_wave_pipelined_matches_per_thread_kernels(nx, monkeypatch):
 @pytest.mark.parametrize("shape", [1, 2])
 @pytest.mark.parametrize("nx", [64, 128, 256, 384, 512, 1024, 2048])
 def test_alternative_pipeline_shapes_match(nx, shape, monkeypatch):
-    """The autotuner's alternative pipeline shapes of the slice step (shape 1: one-warp row groups,
-    4 x 128 column groups; shape 2: early issue with full exchange buffers) give the waves of the
-    per-thread-load kernels bit for bit."""
+    """The autotuner's alternative pipeline shapes of the slice step (shape 1: columns owned by
+    warps at 256 and 512; shape 2: early issue with full exchange buffers, rows of 256 and 2048, columns of
+    384 and 1024) give the waves of the per-thread-load kernels bit for bit."""
     p = specimens.stem_srtio3(nx=nx, ny=nx, na=4, nb=4, nc=6 if nx < 2048 else 2, ns=4, nconf=1, seed=3)
     ref = _stem(p, 0, monkeypatch)
     monkeypatch.setenv("MTB_SHAPE", str(shape | (shape << 2)))
