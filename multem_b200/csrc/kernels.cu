@@ -303,7 +303,7 @@ static void splat_launch(const SplatArgs& a, int islice_0, int n_slice, cudaStre
     const dim3 grid(a.g.ny / SPLAT_TY, a.g.nx / (SPLAT_WARPS * PX), n_slice * a.n_conf);
     const size_t sm = (size_t)a.n_types * a.nR * (sizeof(float4) + sizeof(float2));
     MTB_CUDA(cudaFuncSetAttribute(splat_kernel<PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    launch_early(splat_kernel<PX>, grid, SPLAT_THREADS, sm, s, a, islice_0, n_slice);
+    launch_early(true, splat_kernel<PX>, grid, SPLAT_THREADS, sm, s, a, islice_0, n_slice);
     g_launches++;
 }
 
@@ -414,7 +414,7 @@ __global__ void det_reduce_kernel(const double* __restrict__ partial, int nprobe
 void launch_det_reduce(const double* partial, int nprobe, int n_tiles, int n_det, const int* scan_index, double w,
                        double* image, int n_scan, cudaStream_t s) {
     const int n = nprobe * n_det;
-    launch_early(det_reduce_kernel, (n + 127) / 128, 128, 0, s, partial, nprobe, n_tiles, n_det, scan_index, w, image, n_scan);
+    launch_early(true, det_reduce_kernel, (n + 127) / 128, 128, 0, s, partial, nprobe, n_tiles, n_det, scan_index, w, image, n_scan);
     g_launches++;
 }
 
@@ -564,7 +564,7 @@ __global__ void ew_accumulate_kernel(const float2* __restrict__ psi, int nx, int
 void launch_ew_accumulate(const float2* psi, int nx, int ny, int ix0, int ix1, int iy0, int iy1, double w,
                           int assign, double* psi_out, double* m2_out, cudaStream_t s, int nwave) {
     dim3 grid((ny + 127) / 128, nx);
-    launch_early(ew_accumulate_kernel, grid, 128, 0, s, psi, nx, ny, ix0, ix1, iy0, iy1, w, assign, psi_out, m2_out, nwave);
+    launch_early(true, ew_accumulate_kernel, grid, 128, 0, s, psi, nx, ny, ix0, ix1, iy0, iy1, w, assign, psi_out, m2_out, nwave);
     g_launches++;
 }
 

@@ -10,8 +10,7 @@
 // start-up overlap: called first, successors that hold their place on an SM cost long passes 2 % and
 // put two CTAs on one SM where a pass has fewer CTAs than there are SMs (exit wave of 8 x 256^2, 5 %
 // slower). Measured over whole runs on one B200: exit wave of 16 x 256^2 1546 -> 1478 us, STEM 128^2
-// x 256 probes 2507 -> 2430 us, HRTEM 8 x 512 x 384 1962 -> 1914 us, STEM 256^2 4403 -> 4344 us, 512^2 and
-// 1024^2 unchanged.
+// x 256 probes 2507 -> 2430 us, HRTEM 8 x 512 x 384 1962 -> 1914 us, STEM 256^2 4403 -> 4344 us.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -25,8 +24,9 @@ namespace mtb {
 __device__ __forceinline__ void previous_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// early = false: an ordinary launch, which starts after its predecessor's end.
 template <class... P, class... A>
-void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+void launch_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -36,7 +36,7 @@ void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     MTB_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
 }
 

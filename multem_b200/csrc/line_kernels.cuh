@@ -298,7 +298,8 @@ __global__ void __launch_bounds__(LineGeom<NX>::THREADS, LinePlan<NX>::B) cols_k
     const int items = tiles * a.nprobe;
     const size_t pstride = (size_t)NX * ldy;
 
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        const int item = items - 1 - it;  // the last wave first (see cols_launch_ld)
         const int b = item / tiles;
         const int ct = item % tiles;
         const int iy = ct * W + c;
@@ -731,7 +732,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     auto issue = [&](int k) {
         if (err_set(a.err)) return;
         last_k = k;
-        const int item = blockIdx.x + k * gridDim.x;
+        const int item = items - 1 - (int)(blockIdx.x + k * gridDim.x);
         unsigned long long* bar = &full[k % NG];
         float2* dst = land0 + (k % NG) * P::LAND;
         fence_proxy_async();
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     const GSync gsync{grp};
     const FSync fsync{grp};
     for (int k = grp; k < K; k += NG) {
-        const int item = blockIdx.x + k * gridDim.x;
+        const int item = items - 1 - (int)(blockIdx.x + k * gridDim.x);  // the last wave first (see cols_launch_ld)
         const int b = item / tiles, ct = item % tiles;
         const int iy = ct * W + c;
         float2* dst = a.out + (size_t)b * pstride + (ct * W + cs) + (size_t)ts * ldy;
@@ -830,6 +831,10 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
 void encode_tile_map(CUtensorMap* map, const float2* base, int nx, int ldy, int nprobe, int w, int boxr, bool swizzle);
 
 // ---------------------------------------------------------------------------------------------
+// Passes over more than 256 MB of waves (200 us and more) are launched the ordinary way: starting early
+// gives them nothing (512^2 x 256 waves) or costs 1 to 3 % (1024^2 x 64).
+inline bool long_pass(int nprobe, int nx, int ny) { return (size_t)nprobe * nx * ny > ((size_t)1 << 25); }
+
 // launch helpers (the per-kernel occupancy caps are function-local statics, initialised once and
 // thread-safe, so engines on several host threads may launch concurrently)
 template <class K>
@@ -861,7 +866,7 @@ static bool rows_pipe_try(const RowArgs& a, int grid_ctas, cudaStream_t s) {
         const int units = (a.nx / RP::LPC) * a.nprobe / S::NG;
         int grid = grid_ctas > 0 ? grid_ctas : cap;
         if (grid > units) grid = units;
-        launch_early(kern, grid, S::GT * S::NG, RP::SMEM, s, a);
+        launch_early(!long_pass(a.nprobe, a.nx, NY), kern, grid, S::GT * S::NG, RP::SMEM, s, a);
         note_launch();
         return true;
     } else {
@@ -886,7 +891,7 @@ static void rows_launch(const RowArgs& a, int grid_ctas, cudaStream_t s) {
     const int items = (a.nx / G::LPC) * a.nprobe;
     int grid = grid_ctas > 0 ? grid_ctas : cap;
     if (grid > items) grid = items;
-    launch_early(rows_kernel<NY, MODE>, grid, G::THREADS, sm, s, a);
+    launch_early(!long_pass(a.nprobe, a.nx, NY), rows_kernel<NY, MODE>, grid, G::THREADS, sm, s, a);
     note_launch();
 }
 
@@ -914,7 +919,7 @@ static bool cols_pipe_try(const ColArgs& a, int grid_ctas, cudaStream_t s) {
         if (grid > items) grid = items;
         CUtensorMap map;
         encode_tile_map(&map, a.in, NX, a.ny, a.nprobe, CP::W, CP::BOXR, S::OWN);
-        launch_early(kern, grid, S::GT * S::NG, CP::SMEM, s, a, map);
+        launch_early(!long_pass(a.nprobe, NX, a.ny), kern, grid, S::GT * S::NG, CP::SMEM, s, a, map);
         note_launch();
         return true;
     } else {
@@ -923,6 +928,9 @@ static bool cols_pipe_try(const ColArgs& a, int grid_ctas, cudaStream_t s) {
     }
 }
 
+// Column passes take the batch's waves from the last to the first, row passes from the first to the last: each
+// pass begins with the waves that its predecessor left in the L2 (126 MB) instead of those that it
+// has evicted.
 template <int NX, int FLAGS, int LDY>
 static void cols_launch_ld(const ColArgs& a, int grid_ctas, cudaStream_t s) {
     using G = LineGeom<NX>;
@@ -940,7 +948,7 @@ static void cols_launch_ld(const ColArgs& a, int grid_ctas, cudaStream_t s) {
     const int items = (a.ny / G::LPC) * a.nprobe;
     int grid = grid_ctas > 0 ? grid_ctas : cap;
     if (grid > items) grid = items;
-    launch_early(cols_kernel<NX, FLAGS, LDY>, grid, G::THREADS, sm, s, a);
+    launch_early(!long_pass(a.nprobe, NX, a.ny), cols_kernel<NX, FLAGS, LDY>, grid, G::THREADS, sm, s, a);
     note_launch();
 }
 

@@ -240,8 +240,8 @@ void wgrad_launch(mtb::conv::WgradArgs a, float* dw, float* db, cudaStream_t st)
     auto kern = mtb::conv::wgrad_kernel<NI>;
     const size_t smem = T::smem(a.im.W);
     MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    mtb::launch_early(kern, dim3((unsigned)splits, (unsigned)itiles, (unsigned)otiles), mtb::conv::THREADS, smem, st, a);
-    mtb::launch_early(mtb::conv::wgrad_finalize_kernel, dim3((unsigned)otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st, a, splits,
+    mtb::launch_early(true, kern, dim3((unsigned)splits, (unsigned)itiles, (unsigned)otiles), mtb::conv::THREADS, smem, st, a);
+    mtb::launch_early(true, mtb::conv::wgrad_finalize_kernel, dim3((unsigned)otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st, a, splits,
                       itiles, NI, dw, db);
 }
 
@@ -323,7 +323,7 @@ mt_status mt_sg_loss(const float* head, const void* x, const float* target, cons
         check_shape(B, 1, 2, H, W);
         if (!head || !x || !target || !dhead || !terms) mtb::fail(MT_ERR_INVALID_ARG, "NULL tensor");
         const int n = B * H * W;
-        mtb::launch_early(surrogate_loss_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, head, (const __nv_bfloat16*)x,
+        mtb::launch_early(true, surrogate_loss_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, head, (const __nv_bfloat16*)x,
                           target, scale, (__nv_bfloat16*)dhead, terms, B, H * W, lambda);
     });
 }
@@ -333,7 +333,7 @@ mt_status mt_sg_adam(float* w, void* w_bf16, const float* g, float* m, float* v,
     return run([&] {
         if (n <= 0 || step <= 0) mtb::fail(MT_ERR_INVALID_ARG, "bad Adam arguments");
         const float c1 = 1.0f - std::pow(b1, (float)step), c2 = 1.0f - std::pow(b2, (float)step);
-        mtb::launch_early(adam_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, w, (__nv_bfloat16*)w_bf16, g, m, v, n,
+        mtb::launch_early(true, adam_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, w, (__nv_bfloat16*)w_bf16, g, m, v, n,
                           lr, b1, b2, eps, c1, c2);
     });
 }
@@ -344,7 +344,7 @@ mt_status mt_sg_pool2(const void* in, void* out, int B, int C, int H, int W, flo
         if (H % 2 || W % 2) mtb::fail(MT_ERR_INVALID_ARG, "pooling needs even H and W");
         if (!in || !out) mtb::fail(MT_ERR_INVALID_ARG, "NULL tensor");
         const size_t n = (size_t)B * C * (H / 2) * (W / 2);
-        mtb::launch_early(pool2_kernel, elem_grid(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+        mtb::launch_early(true, pool2_kernel, elem_grid(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)in,
                           (__nv_bfloat16*)out, B * C, H, W, scale);
     });
 }
@@ -354,7 +354,7 @@ mt_status mt_sg_upsample2(const void* in, void* out, int B, int C, int H, int W,
         check_shape(B, C, 1, 2 * H, 2 * W);
         if (!in || !out) mtb::fail(MT_ERR_INVALID_ARG, "NULL tensor");
         const size_t n = (size_t)B * C * (2 * H) * (2 * W);
-        mtb::launch_early(upsample2_kernel, elem_grid(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+        mtb::launch_early(true, upsample2_kernel, elem_grid(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)in,
                           (__nv_bfloat16*)out, B * C, H, W, scale);
     });
 }
@@ -363,7 +363,7 @@ mt_status mt_sg_add(const void* a, const void* b, void* out, long long n, void* 
     return run([&] {
         if (n < 0 || (n > 0 && (!a || !b || !out))) mtb::fail(MT_ERR_INVALID_ARG, "bad add arguments");
         if (n == 0) return;
-        mtb::launch_early(add_kernel, elem_grid((size_t)n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)a,
+        mtb::launch_early(true, add_kernel, elem_grid((size_t)n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)a,
                           (const __nv_bfloat16*)b, (__nv_bfloat16*)out, (size_t)n);
     });
 }
