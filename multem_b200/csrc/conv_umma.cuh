@@ -345,7 +345,7 @@ struct ConvTile {
 // operand, 40 cycles each with 32 channels, epilogue 3 k, or 7-10 k over a cluster), which three CTAs
 // per SM overlap (two: 44 us, four: 37 us for the first layer below). Measured on one B200: 16 images of
 // 32 -> 32 channels at 128 x 128, forward 39 us and data gradient 43 us (im2col through memory and a
-// GEMM: 205 us each); 32 images of 256 -> 256 channels at 4 x 4, 15 us (43 us).
+// GEMM: 205 us each); 32 images of 256 -> 256 channels at 4 x 4, forward 15 us.
 template <int BN, int MT, bool DGRAD>
 __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
     using T = ConvTile<BN, MT>;

@@ -514,7 +514,7 @@ void Engine::pack_atoms(const AtomsF& A, std::vector<float4>& at) const {
 
 // Host part of nb consecutive configurations from c on. Displacements leave z alone, so everything but
 // the displaced atoms is the first one's; the host generator's draws, each configuration's from seeds of
-// its own, are made by one thread per configuration (eight of 2304 atoms: 1.0 ms in turn).
+// its own, are made by one thread per configuration (HRTEM of 8 x 2304 atoms: 2355 -> 1945 us a run).
 void Engine::prepare_batch_host(ConfData* cds, int c, int nb, ConfStage* st) {
     prepare_conf_host(cds[0], c, st[0]);
     if (m_.pn_z) {
@@ -956,7 +956,7 @@ std::vector<char> Engine::graph_signature(const ConfData& cd) const {
 // run_conf as a CUDA graph: the first run of a launch sequence with its arguments (same slot buffers,
 // slice count, thickness map and probe defocus) is launched directly, the second is captured, and
 // that graph is replayed for every later one. A capture and instantiation cost more than they save
-// where nothing follows (a single call of one batch: 16 launches directly 140 us, captured 340 us).
+// where nothing follows (a single call of one batch of 16 launches: 215 us directly, 344 us captured).
 // The line-pass autotuner runs before the capture (it times launches and waits for them).
 void Engine::run_conf_graph(ConfData* const* cds, int nb, ConfGraph& g) {
     if (tune_) tune(*cds[0]);
@@ -1047,9 +1047,8 @@ void Engine::run_conf_batch(ConfData* const* cds, int nb) {
 // timed launches each, twice over): the row pass and the column pass of the slice step in each variant
 // (per-thread loads; bulk-copy fed; bulk-copy fed in the alternative pipeline shapes 1 and 2 of
 // RowPipeShape and ColPipeShape, where a length has them), keeping the fastest of each; then, for STEM
-// batches of at least 16
-// probes, the chosen step at the full and at half the batch, keeping the batch with the lower
-// time per probe. Every variant computes the same transforms with the same rounding, so the
+// batches of at least 16 probes, the chosen step at the full and at half the batch, keeping the batch with
+// the lower time per probe. Every variant computes the same transforms with the same rounding, so the
 // choice changes only the speed (the FP64 detector partials of other tile widths are added in
 // another order).
 Engine::Tuning Engine::tune_passes(int nprobe, ConfData& cd) {
