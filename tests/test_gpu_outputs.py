@@ -1,0 +1,68 @@
+"""Row-major results (mt_engine_run_rows) against the column-major ones of the same engine, over runs that are
+launched directly, captured and replayed; and the potential splat at its tile heights and footprints."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from multem_b200 import api, capi, specimens
+from oracle import multislice as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _wave(nx, ny, sim, coh=0):
+    p = specimens.hrtem_si001(nx=nx, ny=ny, na=2, nb=2, nc=1)
+    p.simulation_type, p.pn_nconf, p.pn_seed, p.pn_coh_contrib = sim, 3, 4, coh
+    return p
+
+
+def _stem(scan_type, coh=0):
+    p = specimens.stem_srtio3(nx=128, ny=128, na=2, nb=2, nc=2, ns=5, nconf=2, seed=3)
+    p.scanning_type, p.pn_coh_contrib = scan_type, coh
+    p.scanning_ye = p.scanning_y0 + 0.6 * (p.scanning_xe - p.scanning_x0)  # 5 x 3 probes
+    return p
+
+
+# 1024 x 512 waves (8 MB) take the threaded copy; a cropped window of odd sides; diffraction with the
+# coherent contribution (squared on the host); area, line and coherent scans
+@pytest.mark.parametrize("name", ["large", "window", "ed_coh", "stem", "stem_line", "stem_coh"])
+def test_row_major_results_are_the_column_major_ones_transposed(name):
+    p = {"large": lambda: _wave(1024, 512, 52), "window": lambda: _wave(128, 64, 52), "ed_coh": lambda: _wave(128, 64, 31, 1),
+         "stem": lambda: _stem(2), "stem_line": lambda: _stem(1), "stem_coh": lambda: _stem(2, 1)}[name]()
+    if name == "window":
+        p.output_area_ix_0, p.output_area_ix_e, p.output_area_iy_0, p.output_area_iy_e = 11, 78, 5, 40
+    e = api.Engine(p)
+    buf = api.OutputBuffers(e.dims)
+    capi.check(e.lib.mt_engine_run(e.h, C.byref(buf.c)))
+    ref = buf.to_dict()
+    for _ in range(4):  # captured on the second run, replayed from then on
+        out = e.run()
+        assert out["dx"] == ref["dx"] and out["dy"] == ref["dy"]
+        for k in ("x", "y", "thick"):
+            np.testing.assert_array_equal(out[k], ref[k])
+        for a, b in zip(out["data"], ref["data"], strict=True):
+            assert a.keys() == b.keys()
+            for k in a:
+                for u, v in zip(a[k], b[k], strict=True) if isinstance(a[k], list) else [(a[k], b[k])]:
+                    assert u.shape == v.shape and u.dtype == v.dtype and u.flags.c_contiguous
+                    np.testing.assert_array_equal(u, v)
+    e.close()
+
+
+# one slice: 2, 4 and 8 pixels per thread (tiles of 64 x 32: 2 to 2048), square and not; a single unit cell's
+# footprints reach across the cell more than once (every periodic image), larger cells' do not
+@pytest.mark.parametrize("nx,ny,na", [(64, 64, 1), (128, 64, 1), (512, 1024, 4), (1024, 1024, 4), (2048, 2048, 4)])
+def test_potential_at_tile_heights_and_wide_footprints(nx, ny, na):
+    p = specimens.stem_srtio3(nx=nx, ny=ny, na=na, nb=na, nc=2, ns=1, nconf=1, seed=2)
+    p.pn_model = 1
+    V = api.ilc_projected_potential(None, p, 1, 1).T
+    grid = O.Grid(nx, ny, p.spec_lx, p.spec_ly)
+    Z, xyz = api.specimen_atoms(p, 1)
+    s = api.specimen_slices(p, 1)
+    i = slice(s["iatom_0"][1], s["iatom_e"][1] + 1)
+    tabs = {int(z): O.atom_table(int(z), min(grid.dRx, grid.dRy)) for z in np.unique(Z)}
+    ref = O.projected_potential(grid, xyz[i, :2], Z[i], np.ones(len(Z[i])), tabs)
+    # positions are floats: x rounded by 2^-24 of 16 A or 1e-6 A, against distances from 0.03 A (a pixel) on,
+    # where the potential falls about as 1/R: 3e-5 at the nearest pixels, less in the norm
+    assert np.linalg.norm(V - ref) < 3e-5 * np.linalg.norm(ref)
