@@ -156,7 +156,7 @@ __device__ __forceinline__ long long pixel_offset(const Image& im, int C, int b0
 }
 
 __device__ __forceinline__ uint16_t ld16(const __nv_bfloat16* p) {
-    return __ldg(reinterpret_cast<const unsigned short*>(p));
+    return *reinterpret_cast<const unsigned short*>(p);
 }
 
 // 8 channels of a pixel packed in order.
@@ -266,7 +266,7 @@ __device__ __forceinline__ void weights8(const __nv_bfloat16* w, int row, int nr
         if (vec) {
 #pragma unroll
             for (int i = 0; i < 9; i++) {
-                const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + i);
+                const uint4 u = reinterpret_cast<const uint4*>(p)[i];
                 h[4 * i] = u.x, h[4 * i + 1] = u.y, h[4 * i + 2] = u.z, h[4 * i + 3] = u.w;
             }
         } else {
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
         for (int c0 = cfirst; c0 < BN; c0 += cstep) {
             float bias[16];
 #pragma unroll
-            for (int j = 0; j < 16; j++) bias[j] = a.bias && n0 + c0 + j < a.Cout ? __ldg(a.bias + n0 + c0 + j) : 0.0f;
+            for (int j = 0; j < 16; j++) bias[j] = a.bias && n0 + c0 + j < a.Cout ? a.bias[n0 + c0 + j] : 0.0f;
             uint32_t r[16];
             tmem_ld16(taddr + (unsigned)c0, r);
             if (o == kNoPixel) continue;
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
             for (int z = 1; z < 8; z++)
                 if (z < a.ksplit) v[0] += q[z].x, v[1] += q[z].y, v[2] += q[z].z, v[3] += q[z].w;
             if (n >= a.Cout) continue;
-            const float bias = a.bias ? __ldg(a.bias + n) : 0.0f;
+            const float bias = a.bias ? a.bias[n] : 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const long long o = pixel_offset(a.im, a.Cout, b0, r0, p + j);
@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
 // order. The CTA row i = Cin does the bias. With infinities or NaN in the tile's inputs the sums run
 // over the image pixels themselves (rows strided over the warps).
 __global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, int splits, int itiles, int NI,
-                                                             float* __restrict__ dw, float* __restrict__ db) {
+                                                             float* dw, float* db) {
     __shared__ float s[8][3][32];
     next_may_start();
     previous_done();
@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, 
 #pragma unroll 4
         for (int k = warp; k < splits; k += 8)
 #pragma unroll
-            for (int t = 0; t < 3; t++) acc[t] += __ldg(p + k * split + t * tap);
+            for (int t = 0; t < 3; t++) acc[t] += p[k * split + t * tap];
     }
     if (__syncthreads_or(special)) {
         const int H = a.im.H, W = a.im.W;

@@ -398,8 +398,8 @@ void launch_cols(int nx, int flags, const ColArgs& a, int grid_ctas, cudaStream_
 
 // =============================================================================================
 // Detector reduction: one thread per (probe, detector); tiles summed in order (deterministic).
-__global__ void det_reduce_kernel(const double* __restrict__ partial, int nprobe, int n_tiles, int n_det,
-                                  const int* __restrict__ scan_index, double w, double* __restrict__ image,
+__global__ void det_reduce_kernel(const double* partial, int nprobe, int n_tiles, int n_det,
+                                  const int* scan_index, double w, double* image,
                                   int n_scan) {
     previous_done();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -528,9 +528,9 @@ void launch_coh_detect(const float2* coh, int n_thk, int n_scan, const ColArgs& 
 
 // EW output accumulation with fft-shift and crop (add_scale_crop_shift_2d /
 // add_scale_square_crop_shift_2d / assign_crop_shift_2d, src/cgpu_fcns.cuh:1681-1780).
-__global__ void ew_accumulate_kernel(const float2* __restrict__ psi, int nx, int ny, int ix0, int ix1, int iy0,
-                                     int iy1, double w, int assign, double* __restrict__ psi_out,
-                                     double* __restrict__ m2_out, int nwave) {
+__global__ void ew_accumulate_kernel(const float2* psi, int nx, int ny, int ix0, int ix1, int iy0,
+                                     int iy1, double w, int assign, double* psi_out,
+                                     double* m2_out, int nwave) {
     previous_done();
     const int iy = blockIdx.x * blockDim.x + threadIdx.x;
     const int ix = blockIdx.y;

@@ -6,6 +6,10 @@
 // kernel that calls neither behaves as ever. Since every early kernel waits for its predecessor's end
 // before its own, the order holds along the whole stream.
 //
+// What an early kernel reads may be written while it is resident, so it is read with ordinary loads only:
+// no __ldg, which wants memory that nothing writes for as long as the kernel runs, and no __restrict__, which
+// makes such loads of plain ones and lets the compiler move them above previous_done().
+//
 // The passes of the slice loop call next_may_start() as their last act, so that only launch latency and
 // start-up overlap: called first, successors that hold their place on an SM cost long passes 2 % and
 // put two CTAs on one SM where a pass has fewer CTAs than there are SMs (exit wave of 8 x 256^2, 5 %

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(LineGeom<NY>::THREADS, LinePlan<NY>::B) rows_k
         } else {
             const float2* Tr = a.trans + (size_t)b * a.trans_stride + (size_t)ix * NY;
 #pragma unroll
-            for (int i = 0; i < E; i++) x[i] = cmul(x[i], __ldg(&Tr[reg_pos<NY, G::RL>(i, t)]));
+            for (int i = 0; i < E; i++) x[i] = cmul(x[i], Tr[reg_pos<NY, G::RL>(i, t)]);
             line_fft<NY, true, -1>(x, buf, twF, t, sync);
 #pragma unroll
             for (int i = 0; i < E; i++) a.out[off + reg_pos<NY, G::R1>(i, t)] = x[i];
@@ -224,7 +224,7 @@ __device__ __forceinline__ double det_pixels(const ColArgs& a, const float2 (&x)
         for (int i = 0; i < G::E; i++) {
             const int ix = reg_pos<NX, G::RL>(i, t);
             const float v2 = __fadd_rn(__fmul_rn(x[i].x, x[i].x), __fmul_rn(x[i].y, x[i].y));
-            acc += (double)__fmul_rn(__ldg(m + (size_t)ix * a.g.ny), v2);
+            acc += (double)__fmul_rn(m[(size_t)ix * a.g.ny], v2);
         }
         return acc;
     }
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(LineGeom<NX>::THREADS, LinePlan<NX>::B) cols_k
             if constexpr (FLAGS & COL_P2) {
                 const float2* p2 = a.P2 + iy;
 #pragma unroll
-                for (int i = 0; i < E; i++) x[i] = cmul(x[i], __ldg(p2 + (size_t)reg_pos<NX, G::RL>(i, t) * a.g.ny));
+                for (int i = 0; i < E; i++) x[i] = cmul(x[i], p2[(size_t)reg_pos<NX, G::RL>(i, t) * a.g.ny]);
             }
         }
         if constexpr (DET) {
@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
             if constexpr (FLAGS & COL_P2) {
                 const float2* p2 = a.P2 + iy;
 #pragma unroll
-                for (int i = 0; i < E; i++) x[i] = cmul(x[i], __ldg(p2 + (size_t)reg_pos<NX, G::RL>(i, t) * a.g.ny));
+                for (int i = 0; i < E; i++) x[i] = cmul(x[i], p2[(size_t)reg_pos<NX, G::RL>(i, t) * a.g.ny]);
             }
         }
         if constexpr (DET) {

@@ -35,9 +35,9 @@ __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162f
 // dn = (yh - t) / s_b:
 //   loss = dn^2 + lambda * (e - |dn|)^2   (the error target is not differentiated)
 // gradients (scaled by 1/n) go to dhead as BF16; per-pixel losses to `terms` for a fixed-order sum.
-__global__ void surrogate_loss_kernel(const float* __restrict__ head, const __nv_bfloat16* __restrict__ x,
-                                      const float* __restrict__ t, const float* __restrict__ scale,
-                                      __nv_bfloat16* __restrict__ dhead, float* __restrict__ terms, int B, int HW,
+__global__ void surrogate_loss_kernel(const float* head, const __nv_bfloat16* x,
+                                      const float* t, const float* scale,
+                                      __nv_bfloat16* dhead, float* terms, int B, int HW,
                                       float lambda) {
     mtb::next_may_start();
     mtb::previous_done();
@@ -56,8 +56,8 @@ __global__ void surrogate_loss_kernel(const float* __restrict__ head, const __nv
 }
 
 // Adam step on FP32 master weights; writes the BF16 copy the kernels read.
-__global__ void adam_kernel(float* __restrict__ wm, __nv_bfloat16* __restrict__ wb, const float* __restrict__ g,
-                            float* __restrict__ m, float* __restrict__ v, int n, float lr, float b1, float b2, float eps,
+__global__ void adam_kernel(float* wm, __nv_bfloat16* wb, const float* g,
+                            float* m, float* v, int n, float lr, float b1, float b2, float eps,
                             float c1, float c2) {
     mtb::next_may_start();
     mtb::previous_done();
@@ -75,7 +75,7 @@ __global__ void adam_kernel(float* __restrict__ wm, __nv_bfloat16* __restrict__ 
 
 // 2 x 2 block sum times `scale` ([B*C, H, W] -> [B*C, H/2, W/2]): average pooling with scale 1/4,
 // the gradient of nearest-neighbour upsampling with scale 1.
-__global__ void pool2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int planes, int H,
+__global__ void pool2_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, int planes, int H,
                              int W, float scale) {
     mtb::next_may_start();
     mtb::previous_done();
@@ -92,7 +92,7 @@ __global__ void pool2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16
 
 // Nearest-neighbour 2x upsampling times `scale` ([B*C, H, W] -> [B*C, 2H, 2W]): upsampling with
 // scale 1, the gradient of average pooling with scale 1/4.
-__global__ void upsample2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int planes,
+__global__ void upsample2_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, int planes,
                                  int H, int W, float scale) {
     mtb::next_may_start();
     mtb::previous_done();
@@ -105,8 +105,8 @@ __global__ void upsample2_kernel(const __nv_bfloat16* __restrict__ in, __nv_bflo
     }
 }
 
-__global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
-                           __nv_bfloat16* __restrict__ out, size_t n) {
+__global__ void add_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b,
+                           __nv_bfloat16* out, size_t n) {
     mtb::next_may_start();
     mtb::previous_done();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
