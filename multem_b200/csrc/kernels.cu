@@ -302,7 +302,10 @@ template <int PX>
 static void splat_launch(const SplatArgs& a, int islice_0, int n_slice, cudaStream_t s) {
     const dim3 grid(a.g.ny / SPLAT_TY, a.g.nx / (SPLAT_WARPS * PX), n_slice * a.n_conf);
     const size_t sm = (size_t)a.n_types * a.nR * (sizeof(float4) + sizeof(float2));
-    MTB_CUDA(cudaFuncSetAttribute(splat_kernel<PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    // the same limit in every launch: it is the kernel's, and other host threads launch with tables of their own size
+    constexpr size_t most = (size_t)kMaxTypes * kMaxKnots * (sizeof(float4) + sizeof(float2));
+    if (sm > most) fail(MT_ERR_UNSUPPORTED, "spline tables larger than the splat's shared memory");
+    MTB_CUDA(cudaFuncSetAttribute(splat_kernel<PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     launch_early(true, splat_kernel<PX>, grid, SPLAT_THREADS, sm, s, a, islice_0, n_slice);
     g_launches++;
 }

@@ -9,6 +9,7 @@ namespace mtb {
 
 constexpr int kMaxDet = 8;
 constexpr int kMaxTypes = 16;
+constexpr int kMaxKnots = 128;  // of a type's potential tables
 
 // Grid_2d<float> fields the kernels use (src/types.cuh:2107-2655).
 struct GridDev {

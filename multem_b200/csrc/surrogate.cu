@@ -137,6 +137,10 @@ void check_shape(int B, int Cin, int Cout, int H, int W) {
         mtb::fail(MT_ERR_INVALID_ARG, "bad convolution shape");
 }
 
+// Shared memory that the convolution kernels may ask for: the same limit in every launch, since it is the
+// kernel's and other host threads launch it with tiles of another size (227 KB less the static variables).
+constexpr int kSmemMax = 232448 - 1024;
+
 constexpr long long kWaitNs = 1000000000ll;  // bound of every wait for the tensor cores (1 s)
 
 // whether every row of w [..][Cin][3][3] (bf16) starts on a 16-byte boundary
@@ -181,7 +185,7 @@ void conv_launch(const mtb::conv::ConvArgs& a, cudaStream_t st) {
     using T = mtb::conv::ConvTile<BN, MT>;
     auto kern = mtb::conv::conv_kernel<BN, MT, DGRAD>;
     const size_t smem = T::smem(a.im.W, a.Cin, a.ksplit);
-    MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)((a.im.total() + T::TM - 1) / T::TM), (unsigned)((a.Cout + BN - 1) / BN), (unsigned)a.ksplit);
     cfg.blockDim = dim3(mtb::conv::THREADS);
@@ -239,7 +243,7 @@ void wgrad_launch(mtb::conv::WgradArgs a, float* dw, float* db, cudaStream_t st)
     a.err = ws.err;
     auto kern = mtb::conv::wgrad_kernel<NI>;
     const size_t smem = T::smem(a.im.W);
-    MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     mtb::launch_early(true, kern, dim3((unsigned)splits, (unsigned)itiles, (unsigned)otiles), mtb::conv::THREADS, smem, st, a);
     mtb::launch_early(true, mtb::conv::wgrad_finalize_kernel, dim3((unsigned)otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st, a, splits,
                       itiles, NI, dw, db);
@@ -288,10 +292,9 @@ mt_status mt_sg_conv3x3_backward_weight(const void* in, const void* dout, const 
         a.wait_ns = kWaitNs;
         // input channels per CTA: the gradient tile is gathered once for each, so as many as the
         // layer has and two stages of shared memory hold
-        constexpr size_t kSmem = 232448 - 1024;
         if (Cin <= 16) wgrad_launch<16>(a, dw, db, st);
         else if (Cin <= 32) wgrad_launch<32>(a, dw, db, st);
-        else if (Cin <= 64 || mtb::conv::WgradTile<128>::smem(W) > kSmem) wgrad_launch<64>(a, dw, db, st);
+        else if (Cin <= 64 || mtb::conv::WgradTile<128>::smem(W) > (size_t)kSmemMax) wgrad_launch<64>(a, dw, db, st);
         else wgrad_launch<128>(a, dw, db, st);
     });
 }
