@@ -14,6 +14,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 
@@ -310,11 +311,23 @@ static void splat_launch(const SplatArgs& a, int islice_0, int n_slice, cudaStre
     g_launches++;
 }
 
-// Slices islice_0 .. islice_0 + n_slice - 1 of the n_conf configurations of `a` in one launch. Taller
-// warps (more pixels per thread) reuse a lane's (y - y_atom)^2 more often; shorter ones where the tiles
-// would leave an SM with less than four CTAs.
+// Slices islice_0 .. islice_0 + n_slice - 1 of the n_conf configurations of `a`, as many configurations per
+// launch as the grid's z extent takes (65535 slices in all). Taller warps (more pixels per thread) reuse a
+// lane's (y - y_atom)^2 more often; shorter ones where the tiles would leave an SM with less than four CTAs.
 void launch_splat(const SplatArgs& a, int islice_0, int n_slice, cudaStream_t s) {
     if (a.g.nx % (SPLAT_WARPS * 8) || a.g.ny % SPLAT_TY) fail(MT_ERR_UNSUPPORTED, "grid must be a multiple of 64 x 32");
+    const int most = std::max(1, 65535 / n_slice);
+    if (a.n_conf > most) {
+        for (int c = 0; c < a.n_conf; c += most) {
+            SplatArgs part = a;
+            part.n_conf = std::min(most, a.n_conf - c);
+            std::copy(a.conf + c, a.conf + c + part.n_conf, part.conf);
+            if (a.trans) part.trans = a.trans + c * a.trans_stride;
+            if (a.V) part.V = a.V + c * a.trans_stride;
+            launch_splat(part, islice_0, n_slice, s);
+        }
+        return;
+    }
     const long long tiles = (long long)(a.g.nx / 64) * (a.g.ny / SPLAT_TY) * n_slice * a.n_conf;
     if (tiles >= 4 * 148) splat_launch<8>(a, islice_0, n_slice, s);
     else if (2 * tiles >= 4 * 148) splat_launch<4>(a, islice_0, n_slice, s);

@@ -55,3 +55,20 @@ def test_batched_configurations_match_one_at_a_time(name, nconf, monkeypatch):
     for k in ref:
         np.testing.assert_array_equal(direct[k], ref[k], err_msg=k)
 
+
+
+def test_batch_of_a_specimen_of_many_slices(monkeypatch):
+    """Eight configurations of more than 8191 slices: more (configuration, slice) pairs than one launch of
+    the potential splat can number (65535)."""
+    from multem_b200 import specimens
+    p = specimens.hrtem_si001(nx=64, ny=64, na=1, nb=1, nc=1)
+    atoms = np.asarray(p.spec_atoms)[:4].copy()
+    atoms[:, 3] = [0.0, 1000.0, 4200.0, 8300.0]
+    p.spec_atoms, p.spec_lz, p.spec_dz, p.potential_slicing = atoms, 8300.0, 1.0, 2
+    p.pn_nconf, p.pn_seed = 8, 3
+    assert len(api.specimen_slices(p, 1)["iatom_0"]) > 8191
+    got = _arrays(api.ilc_multem(None, p))
+    monkeypatch.setenv("MTB_EW_BATCH", "1")
+    ref = _arrays(api.ilc_multem(None, p))
+    for k in ref:
+        np.testing.assert_array_equal(got[k], ref[k], err_msg=k)
