@@ -15,15 +15,13 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <exception>
 #include <map>
 #include <mutex>
-#include <system_error>
-#include <thread>
 #include <tuple>
 
 #include "common.hpp"
 #include "engine.hpp"
+#include "host_threads.hpp"
 
 namespace mtb {
 
@@ -527,8 +525,6 @@ void Engine::prepare_batch_host(ConfData* cds, int c, int nb, ConfStage* st) {
         s.move_atoms(c + b);
         pack_atoms(s.atoms(), st[b].at);
     };
-    std::vector<std::thread> pool;
-    std::vector<std::exception_ptr> failed(nb);
     for (int b = 1; b < nb; b++) {
         const ConfData& first = cds[0];
         ConfData& cd = cds[b];
@@ -543,32 +539,13 @@ void Engine::prepare_batch_host(ConfData* cds, int c, int nb, ConfStage* st) {
         st[b].prop = st[0].prop;
         st[b].n_atoms = st[0].n_atoms;
         st[b].at.clear();
-        if (!host_rng) continue;
-        bool started = false;
-        if (b + 1 < nb && st[0].n_atoms >= 256) {  // the last one is this thread's
-            try {
-                pool.emplace_back([&, b] {
-                    try {
-                        draw(b);
-                    } catch (...) {
-                        failed[b] = std::current_exception();
-                    }
-                });
-                started = true;
-            } catch (const std::system_error&) {  // no more threads: drawn here
-            }
-        }
-        if (!started) {
-            try {
-                draw(b);
-            } catch (...) {
-                failed[b] = std::current_exception();
-            }
-        }
     }
-    for (auto& t : pool) t.join();
-    for (auto& e : failed)
-        if (e) std::rethrow_exception(e);
+    if (!host_rng) return;
+    if (st[0].n_atoms >= 256) {
+        run_threads(nb - 1, [&](int i) { draw(1 + i); });
+    } else {
+        for (int b = 1; b < nb; b++) draw(b);
+    }
 }
 
 // Host part of a configuration's set-up: phonon displacement (host generator), slicing, propagator
@@ -1635,14 +1612,7 @@ void Engine::copy_out(void* dst, const void* src, size_t bytes) {
         if (s) cudaStreamDestroy(s);
         if (e != cudaSuccess) status = e;
     };
-    std::vector<std::thread> pool;
-    pool.reserve(kThreads);
-    try {
-        for (int t = 1; t < kThreads; t++) pool.emplace_back(work, t);
-    } catch (const std::system_error&) {  // no more threads: those that started and this one do it
-    }
-    work(0);
-    for (auto& t : pool) t.join();
+    run_threads(kThreads, work);
     MTB_CUDA((cudaError_t)status.load());
 }
 
