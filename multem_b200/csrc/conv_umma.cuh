@@ -315,7 +315,8 @@ struct ConvArgs {
 template <int BN, int MT>
 struct ConvTile {
     static constexpr int TM = 128 * MT;
-    static constexpr unsigned COLS = tmem_cols(MT * BN);
+    static constexpr int NACC = MT == 1 ? 4 : 1;  // accumulators that take the products in turn
+    static constexpr unsigned COLS = tmem_cols(NACC * MT * BN);
     static __host__ __device__ int seg(int W) { return W + 1 <= TM + 2 ? W + 1 : TM + 2; }  // pixels between taps ky
     static __host__ __device__ int npix(int W) { return TM + 2 + 2 * seg(W); }
     static __host__ __device__ int nplane(int Cin) { return Cin <= 16 ? 2 : KC / 8; }
@@ -340,6 +341,11 @@ struct ConvTile {
 // [n / 8][k][n % 8] for the data gradient, which are the planes that 16-byte pieces of w give without
 // a transposition. Where the tiles alone leave SMs idle, a cluster of ksplit CTAs shares a tile's input
 // channels and adds the partial sums through its shared memory.
+//
+// An accumulator loses about 1.1e-8 of the sum with every MMA that it takes in (the products are aligned to it and
+// cut off), so a sum of n in a row is off by 1.1e-8 n. One pixel tile per CTA therefore spreads its products
+// over four accumulators (channel group x parity of the tap; two for up to 16 channels), added in
+// FP32 by the epilogue; two tiles per CTA, which large batches take, have the tensor memory for one.
 //
 // Bound by the chain of a CTA (about 18 k cycles: weights 3 k, gather 2-5 k, the MMAs' reads of the pixel
 // operand, 40 cycles each with 32 channels, epilogue 3 k, or 7-10 k over a cluster), which three CTAs
@@ -422,18 +428,18 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
             const uint32_t da = desc_lo(smem_u32(st), 16u * npix), db = desc_lo(smem_u32(st + bbytes), DGRAD ? 128u : 16u * BN);
             const unsigned bstride = DGRAD ? 16u * kw : 128u;
             const uint32_t btap = DGRAD ? (BN / 8) * kw : nplane * BN;
-            unsigned acc = kb > 0;
 #pragma unroll 1
             for (int k = 0; k < nplane / 2; k++) {
+                const unsigned acc = kb > 0 || (T::NACC == 1 && k > 0);
+                const unsigned tmem_k = tmem + (T::NACC == 1 ? 0 : 2 * k * BN);
                 const uint32_t dak = da + 2 * k * npix, dbk = db + (DGRAD ? 16 * k : 2 * k * BN);
 #pragma unroll
                 for (int t = 0; t < 9; t++) {
 #pragma unroll
                     for (int m = 0; m < MT; m++)
-                        mma_bf16(tmem + m * BN, desc(dak + (t / 3) * seg + (t % 3) + 128 * m, 128u), desc(dbk + t * btap, bstride),
-                                 id, acc | (t > 0));
+                        mma_bf16(tmem_k + (T::NACC == 1 ? m * BN : (t & 1) * BN), desc(dak + (t / 3) * seg + (t % 3) + 128 * m, 128u),
+                                 desc(dbk + t * btap, bstride), id, acc | (t >= (T::NACC == 1 ? 1 : 2)));
                 }
-                acc = 1u;
             }
             mma_commit(&done[kb & 1]);
         }
@@ -449,6 +455,21 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
     const int row = 128 * mt + 32 * (warp % 4) + lane;
     const int cfirst = MT == 2 ? 0 : 16 * (warp / 4), cstep = MT == 2 ? 16 : 32;
     const unsigned taddr = tmem + ((unsigned)(32 * (warp % 4)) << 16) + (unsigned)(mt * BN);
+    // the sum of the accumulators in use, of 16 columns from c0 on
+    auto sums = [&](int c0, float (&v)[16]) {
+        uint32_t r[16];
+        tmem_ld16(taddr + (unsigned)c0, r);
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
+        if constexpr (T::NACC > 1) {
+#pragma unroll 1
+            for (int i = 1; i < nplane; i++) {
+                tmem_ld16(taddr + (unsigned)(i * BN + c0), r);
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] += __uint_as_float(r[j]);
+            }
+        }
+    };
     if (a.ksplit == 1) {
         const long long o = pixel_offset(a.im, a.Cout, b0, r0, row);
         const size_t obase = (size_t)b0 * a.Cout * hw + (size_t)(o == kNoPixel ? 0 : o);
@@ -457,15 +478,14 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
             float bias[16];
 #pragma unroll
             for (int j = 0; j < 16; j++) bias[j] = a.bias && n0 + c0 + j < a.Cout ? a.bias[n0 + c0 + j] : 0.0f;
-            uint32_t r[16];
-            tmem_ld16(taddr + (unsigned)c0, r);
+            float v[16];
+            sums(c0, v);
             if (o == kNoPixel) continue;
             const size_t at = obase + (size_t)(n0 + c0) * hw;
             const int n = a.Cout - n0 - c0;
-            float v[16];
 #pragma unroll
             for (int j = 0; j < 16; j++) {
-                v[j] = (ok ? __uint_as_float(r[j]) : 0.0f) + bias[j];
+                v[j] = (ok ? v[j] : 0.0f) + bias[j];
                 if (a.relu) v[j] = fmaxf(v[j], 0.0f);
             }
             if (a.out_bf)
@@ -483,10 +503,10 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
         float* part = reinterpret_cast<float*>(stage0);
 #pragma unroll 1
         for (int c0 = cfirst; c0 < BN; c0 += cstep) {
-            uint32_t r[16];
-            tmem_ld16(taddr + (unsigned)c0, r);
+            float v[16];
+            sums(c0, v);
 #pragma unroll
-            for (int j = 0; j < 16; j++) part[(c0 + j) * T::TM + row] = ok ? __uint_as_float(r[j]) : 0.0f;
+            for (int j = 0; j < 16; j++) part[(c0 + j) * T::TM + row] = ok ? v[j] : 0.0f;
         }
         cluster_sync();
         const int quads = T::TM / 4, cols = BN / a.ksplit;

@@ -214,9 +214,14 @@ void conv(mtb::conv::ConvArgs a, cudaStream_t st) {
     auto ctas = [&](int bn) { return tiles * ((a.Cout + bn - 1) / bn); };
     int bn = a.Cout <= 16 ? 16 : a.Cout <= 32 ? 32 : 64;
     while (bn > 16 && ctas(bn) * most < 148) bn /= 2;
+    // K is cut into `parts` at least (over CTAs and accumulators) where that leaves more than two blocks to each CTA
+    const long long m = ((long long)a.im.B * a.im.H * a.im.W + 127) / 128 * ((a.Cout + 255) / 256);
+    const long long parts = (295 + m) / m;
     a.ksplit = 1;
-    while (a.ksplit < most && ctas(bn) * a.ksplit < 148) a.ksplit *= 2;
-    const bool two = ctas(bn) >= 4 * 148;
+    while (a.ksplit < most && (ctas(bn) * a.ksplit < 148 ||
+                               (nkb + a.ksplit - 1) / a.ksplit > std::max<long long>(2, 4 * nkb / parts)))
+        a.ksplit *= 2;
+    const bool two = ctas(bn) >= 4 * 148 && parts == 1;
     switch (bn) {
         case 16: two ? conv_launch<16, 2, DGRAD>(a, st) : conv_launch<16, 1, DGRAD>(a, st); break;
         case 32: two ? conv_launch<32, 2, DGRAD>(a, st) : conv_launch<32, 1, DGRAD>(a, st); break;

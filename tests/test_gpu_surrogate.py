@@ -248,3 +248,21 @@ def test_trained_surrogate_gains_over_the_plain_few_configuration_image():
         assert e_learned < e_plain
         if ok:
             assert e_learned <= 2 * sg.gate
+
+
+# An accumulator of the tensor core loses up to about 1.5e-8 of the sum per product of 16 that it takes in (measured
+# 1.1e-8); small batches spread theirs over four accumulators and, where there are many channels, over CTAs. n: products
+# in a row (a K block of 32 channels gives each accumulator 5 at most); 5e-8 for the FP32 sum and result.
+@pytest.mark.parametrize("B,Cin,Cout,H,W,n", [(32, 32, 32, 32, 32, 5), (32, 32, 64, 16, 16, 5), (32, 64, 32, 32, 32, 10),
+                                               (1, 256, 256, 8, 8, 5), (32, 256, 128, 8, 8, 10), (8, 256, 64, 64, 64, 40),
+                                               (16, 32, 32, 128, 128, 18)])
+def test_convolution_sums_against_64_bits(B, Cin, Cout, H, W, n):
+    torch = pytest.importorskip("torch")
+    lib = capi.load()
+    g = torch.Generator().manual_seed(Cin)
+    x = torch.randn(B, Cin, H, W, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(Cout, Cin, 3, 3, generator=g) * (2 / (9 * Cin)) ** 0.5).to(torch.bfloat16).cuda()
+    y = torch.empty(B, Cout, H, W, device="cuda")
+    capi.check(lib.mt_sg_conv3x3_forward(_p(x), _p(w), None, None, _p(y), B, Cin, Cout, H, W, 0, None))
+    ref = torch.nn.functional.conv2d(x.double(), w.double(), padding=1)
+    assert _rel(y.double(), ref) < 1.5e-8 * n + 5e-8
