@@ -227,9 +227,10 @@ class Engine {
     // group the events of its uploads and of its last run
     cudaStream_t up_stream_ = nullptr;
     cudaEvent_t up_done_[2] = {}, group_done_[2] = {};
-    // device to host copy of a finished result; large ones through pinned pieces by several threads
+    // device to host copy of a finished result; large ones by several threads
     void copy_out(void* dst, const void* src, size_t bytes);
-    void* copy_stage_ = nullptr;
+    void* copy_stage_ = nullptr;      // pinned pieces of an engine that has copied a lot
+    size_t copied_ = 0;               // bytes of large results so far
     void copy_images(double* dst, const double* src, size_t planes, int nx, int ny, int width, bool rows);
     DevBuf<double> d_rows_;           // transposed images
     void run_conf(ConfData& cd);
