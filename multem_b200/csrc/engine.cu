@@ -1570,16 +1570,35 @@ void Engine::write_output(mt_output_multislice* out, bool rows) {
 }
 
 // `planes` images of nx x ny values (`width` doubles each), [ix][iy] on the device, to the host as they
-// are or as rows [iy][ix].
+// are or as rows [iy][ix]. The rows are laid out, as many as fit, where the transmission functions are (the
+// next run fills them anew), so results of any size take no device memory of their own.
 void Engine::copy_images(double* dst, const double* src, size_t planes, int nx, int ny, int width, bool rows) {
-    const size_t n = planes * nx * ny * width;
-    if (rows && nx > 1 && ny > 1) {
-        d_rows_.alloc(n);
-        launch_transpose(src, d_rows_.p, planes, nx, ny, width, stream_);
-        src = d_rows_.p;
+    const size_t row = (size_t)nx * width, n = row * ny;
+    if (!rows || nx <= 1 || ny <= 1) {
+        MTB_CUDA(cudaStreamSynchronize(stream_));
+        copy_out(dst, src, planes * n * sizeof(double));
+        return;
     }
-    MTB_CUDA(cudaStreamSynchronize(stream_));
-    copy_out(dst, src, n * sizeof(double));
+    static_assert(sizeof(*d_trans_.p) == sizeof(double), "the transmission functions as room for results");
+    double* room = reinterpret_cast<double*>(d_trans_.p);
+    size_t cap = d_trans_.n;
+    if (cap < 32 * row) {  // lines of a scan that are long for the grid
+        d_rows_.alloc(32 * row);
+        room = d_rows_.p;
+        cap = d_rows_.n;
+    }
+    auto part = [&](size_t p, size_t np, int iy, int ni) {  // rows iy .. iy + ni - 1 of planes p .. p + np - 1
+        launch_transpose(src + p * n + (size_t)iy * width, room, np, nx, ni, ny, width, stream_);
+        MTB_CUDA(cudaStreamSynchronize(stream_));
+        copy_out(dst + p * n + iy * row, room, np * ni * row * sizeof(double));
+    };
+    if (cap >= n) {
+        for (size_t p = 0; p < planes; p += cap / n) part(p, std::min(cap / n, planes - p), 0, ny);
+    } else {
+        const int ni = (int)(cap / row / 32 * 32);
+        for (size_t p = 0; p < planes; p++)
+            for (int iy = 0; iy < ny; iy += ni) part(p, 1, iy, std::min(ni, ny - iy));
+    }
 }
 
 // Most of the time of a large result goes into the first touch of the caller's pages, so several threads touch

@@ -232,7 +232,7 @@ class Engine {
     void* copy_stage_ = nullptr;      // pinned pieces of an engine that has copied a lot
     size_t copied_ = 0;               // bytes of large results so far
     void copy_images(double* dst, const double* src, size_t planes, int nx, int ny, int width, bool rows);
-    DevBuf<double> d_rows_;           // transposed images
+    DevBuf<double> d_rows_;           // transposed rows that the transmission functions have no room for
     void run_conf(ConfData& cd);
     // the splats of nb configurations (into consecutive transmission blocks) and their slice loop
     // (nb > 1: exit-wave family only, configurations with identical slicing)

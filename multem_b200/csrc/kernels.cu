@@ -586,27 +586,27 @@ void launch_ew_accumulate(const float2* psi, int nx, int ny, int ix0, int ix1, i
 
 // 32 x 32 tiles through shared memory, both sides coalesced.
 template <class T>
-__global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny) {
+__global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny, int ld) {
     __shared__ T tile[32][33];
-    const size_t plane = (size_t)blockIdx.z * nx * ny;
+    const size_t sp = (size_t)blockIdx.z * nx * ld, dp = (size_t)blockIdx.z * nx * ny;
     const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
     const int iy0 = blockIdx.x * 32, ix0 = blockIdx.y * 32;
     for (int r = ly; r < 32; r += 8)
-        if (ix0 + r < nx && iy0 + lx < ny) tile[r][lx] = src[plane + (size_t)(ix0 + r) * ny + iy0 + lx];
+        if (ix0 + r < nx && iy0 + lx < ny) tile[r][lx] = src[sp + (size_t)(ix0 + r) * ld + iy0 + lx];
     __syncthreads();
     for (int r = ly; r < 32; r += 8)
-        if (iy0 + r < ny && ix0 + lx < nx) dst[plane + (size_t)(iy0 + r) * nx + ix0 + lx] = tile[lx][r];
+        if (iy0 + r < ny && ix0 + lx < nx) dst[dp + (size_t)(iy0 + r) * nx + ix0 + lx] = tile[lx][r];
 }
 
-void launch_transpose(const double* src, double* dst, size_t planes, int nx, int ny, int width, cudaStream_t s) {
-    const size_t n = (size_t)nx * ny * width;
+void launch_transpose(const double* src, double* dst, size_t planes, int nx, int ny, int ld, int width, cudaStream_t s) {
+    const size_t sn = (size_t)nx * ld * width, dn = (size_t)nx * ny * width;
     for (size_t p = 0; p < planes; p += 65535) {
         const dim3 grid((unsigned)((ny + 31) / 32), (unsigned)((nx + 31) / 32), (unsigned)std::min<size_t>(65535, planes - p));
         if (width == 2)
-            transpose_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const double2*>(src + p * n),
-                                                  reinterpret_cast<double2*>(dst + p * n), nx, ny);
+            transpose_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const double2*>(src + p * sn),
+                                                  reinterpret_cast<double2*>(dst + p * dn), nx, ny, ld);
         else
-            transpose_kernel<<<grid, 256, 0, s>>>(src + p * n, dst + p * n, nx, ny);
+            transpose_kernel<<<grid, 256, 0, s>>>(src + p * sn, dst + p * dn, nx, ny, ld);
         g_launches++;
         MTB_CUDA(cudaGetLastError());
     }

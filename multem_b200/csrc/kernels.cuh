@@ -149,8 +149,8 @@ void launch_coh_detect(const float2* coh, int n_thk, int n_scan, const ColArgs& 
 void launch_ew_accumulate(const float2* psi, int nx, int ny, int ix0, int ix1, int iy0, int iy1, double w,
                           int assign, double* psi_out, double* m2_out, cudaStream_t s, int nwave = 1);
 
-// dst[plane][iy][ix] = src[plane][ix][iy], `width` (1 or 2) doubles per value.
-void launch_transpose(const double* src, double* dst, size_t planes, int nx, int ny, int width, cudaStream_t s);
+// dst[plane][iy][ix] = src[plane][ix][iy], iy < ny, `width` (1 or 2) doubles per value; lines of ld values in src.
+void launch_transpose(const double* src, double* dst, size_t planes, int nx, int ny, int ld, int width, cudaStream_t s);
 
 // Device-side counters of this library's launches (for reporting).
 long long launches_issued();

@@ -51,6 +51,37 @@ def test_row_major_results_are_the_column_major_ones_transposed(name):
     e.close()
 
 
+# results against the room of the transmission functions, in doubles: three thicknesses of complex planes in pieces of
+# one or two planes (one slice per thickness: 3 x 64 x 64 against 3 x 128 x 64 doubles), one plane in strips of rows
+# (one slice), a scan of longer lines than one slice has room for
+@pytest.mark.parametrize("name", ["planes", "strips", "scan"])
+def test_row_major_results_take_no_device_memory(name):
+    p = _wave(64, 64, 52) if name != "scan" else _stem(2)
+    p.pn_nconf, p.pn_model = 1, 1
+    if name == "planes":
+        p.thick_type, p.thick = 2, [1.0, 2.3, 3.7]
+    elif name == "strips":
+        p.interaction_model = 2
+    else:
+        p.nx = p.ny = 64
+        p.interaction_model, p.scanning_ns, p.scanning_square_pxs = 2, 130, 1
+    e = api.Engine(p)
+    buf = api.OutputBuffers(e.dims)
+    for _ in range(3):
+        capi.check(e.lib.mt_engine_run(e.h, C.byref(buf.c)))
+    ref, n = buf.to_dict(), C.c_longlong()
+    e.lib.mt_device_alloc_count(C.byref(n))
+    before = n.value
+    for _ in range(2):
+        for a, b in zip(e.run()["data"], ref["data"], strict=True):
+            for k in a:
+                for u, v in zip(a[k], b[k], strict=True) if isinstance(a[k], list) else [(a[k], b[k])]:
+                    np.testing.assert_array_equal(u, v)
+    e.lib.mt_device_alloc_count(C.byref(n))
+    assert n.value - before == (1 if name == "scan" else 0)  # 32 lines of the scan: more than one slice of 64 x 64
+    e.close()
+
+
 def test_large_results_of_first_and_later_runs():
     """An engine copies its first 256 MB of large results into pages that several threads have touched, later ones through
     pinned pieces: 48 MB a run, in pieces that do not divide the results of a cropped window."""
