@@ -310,9 +310,10 @@ mt_status mt_engine_launch_count(mt_engine* eng, long long* n);
 mt_status mt_engine_pass_variants(mt_engine* eng, int* variants);
 /* The autotuner's full choice for the engine's grid (no counterpart in the reference, whose FFT
  * shapes come from cuFFT plans, src/fft.cuh:364-478): the variant of the row and of the column
- * pass of the slice step (0 per-thread loads, 1 bulk-copy fed, 2 and 3 bulk-copy fed in the two
- * alternative pipeline shapes: narrower groups, and early issue with full exchange buffers) and the
- * probes per launch; valid after a run. */
+ * pass of the slice step (0 per-thread loads, 1 bulk-copy fed, 2 and 3 bulk-copy fed in an
+ * alternative pipeline shape: columns owned by warps, 256 and 512 points; early issue with full
+ * exchange buffers, rows of 256 and 2048 and columns of 384 and 1024) and the probes per launch; valid
+ * after a run. */
 mt_status mt_engine_tuning(mt_engine* eng, int* rows_variant, int* cols_variant, int* probes_per_launch);
 /* Device timing (no counterpart in the reference): with timing on, each run records CUDA events on
  * the engine's stream around the whole run and around every line-pass launch. mt_engine_timing

@@ -1019,20 +1019,26 @@ void Engine::run_conf_batch(ConfData* const* cds, int nb) {
     if (m_.is_scanning()) run_stem(*cds[0]); else run_ew(cds, nb);
 }
 
-// Autotuner of the line passes. For each (nx, ny, allocated probes per launch) the process times,
-// once, on this engine's probe buffer, transmission function and propagator (one warm-up and three
-// timed launches each, twice over): the row pass and the column pass of the slice step in each variant
-// (per-thread loads; bulk-copy fed; bulk-copy fed in the alternative pipeline shapes 1 and 2 of
-// RowPipeShape and ColPipeShape, where a length has them), keeping the fastest of each; then, for STEM
-// batches of at least 16 probes, the chosen step at the full and at half the batch, keeping the batch with
-// the lower time per probe. Every variant computes the same transforms with the same rounding, so the
-// choice changes only the speed (the FP64 detector partials of other tile widths are added in
-// another order).
+// Autotuner of the line passes. For each (nx, ny, allocated probes per launch, shared transmission functions or not)
+// the process times, once, on this engine's probe buffer, transmission functions and propagator, the row pass
+// and the column pass of the slice step in each variant that the lengths have (per-thread loads; bulk-copy
+// fed; bulk-copy fed in an alternative pipeline shape), twice over, and keeps the fastest of each; then,
+// for STEM batches of at least 16 probes, the chosen step at the full and at half the batch, keeping the
+// batch with the lower time per probe. Every variant computes the same transforms with the same
+// rounding, so the choice changes only the speed (the FP64 detector partials of other tile widths are
+// added in another order).
+//
+// Passes over more than 8 MB of waves are timed by themselves, three launches after a first. Shorter ones, a few
+// microseconds each, are timed as they run, rows and columns in turn, over eight steps: what tells the variants apart
+// there is how a pass starts while the other one ends. (Columns, change per slice from per-thread loads to
+// bulk-copy fed on one B200: one wave of 1024 x 64 to 1024^2 -3 to -5 us of 17 to 30, 8 of 128 x 128 +0.6 of 9, of 256 x 256
+// +0.7 of 14, 3 of 512^2 +1.9 of 22.)
 Engine::Tuning Engine::tune_passes(int nprobe, ConfData& cd) {
     static std::mutex mu;
-    static std::map<std::tuple<int, int, int>, Tuning> chosen;
+    static std::map<std::tuple<int, int, int, bool>, Tuning> chosen;
     const int nx = m_.grid.nx, ny = m_.grid.ny;
-    const auto key = std::make_tuple(nx, ny, nprobe);
+    const bool one_trans = shared_trans();
+    const auto key = std::make_tuple(nx, ny, nprobe, one_trans);
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = chosen.find(key);
@@ -1043,20 +1049,21 @@ Engine::Tuning Engine::tune_passes(int nprobe, ConfData& cd) {
     cudaEvent_t a, b;
     MTB_CUDA(cudaEventCreate(&a));
     MTB_CUDA(cudaEventCreate(&b));
-    auto time_of = [&](auto launch) {
+    auto time_of = [&](int n, auto launch) {
         launch();
         MTB_CUDA(cudaEventRecord(a, stream_));
-        for (int i = 0; i < 3; i++) launch();
+        for (int i = 0; i < n; i++) launch();
         MTB_CUDA(cudaEventRecord(b, stream_));
         MTB_CUDA(cudaEventSynchronize(b));
         float ms = 0;
         MTB_CUDA(cudaEventElapsedTime(&ms, a, b));
-        return ms;
+        return ms / n;
     };
     RowArgs ra{};
     ra.in = d_psi_.p;
     ra.out = d_psi_.p;
     ra.trans = d_trans_.p;
+    ra.trans_stride = one_trans ? 0 : (size_t)spec_->slices().size() * nxy;
     ra.nx = nx;
     ra.scale = 1.0f;
     ra.wait_ns = wait_ns_;
@@ -1070,37 +1077,44 @@ Engine::Tuning Engine::tune_passes(int nprobe, ConfData& cd) {
     ca.det_w = col_det_width(nx);
     ca.wait_ns = wait_ns_;
     const int step = COL_LOAD | COL_PROP | COL_INVERSE | COL_STORE;
-    // variant v: 0 per-thread loads, 1 bulk-copy fed, 2 and 3 bulk-copy fed in the alternative
-    // pipeline shapes 1 and 2 (a shape that does not fit this length runs the default one)
-    auto rows_t = [&](int v, int nb) {
+    auto rows_v = [&](int v, int nb) {
         ra.nprobe = nb;
         ra.err = v ? d_err_.p : nullptr;
         ra.shape = v > 1 ? v - 1 : 0;
-        return time_of([&] { launch_rows(ny, ROW_STEP, ra, 0, stream_); });
+        launch_rows(ny, ROW_STEP, ra, 0, stream_);
     };
-    auto cols_t = [&](int v, int nb) {
+    auto cols_v = [&](int v, int nb) {
         ca.nprobe = nb;
         ca.err = v ? d_err_.p : nullptr;
         ca.shape = v > 1 ? v - 1 : 0;
-        return time_of([&] { launch_cols(nx, step, ca, 0, stream_); });
+        launch_cols(nx, step, ca, 0, stream_);
     };
-    constexpr int NV = 4;
-    float tr[NV], tc[NV];
+    const bool brief = nprobe * nxy <= ((size_t)1 << 20);
+    auto rows_t = [&](int v, int nb) {
+        return brief ? time_of(8, [&] { rows_v(v, nb); cols_v(0, nb); }) : time_of(3, [&] { rows_v(v, nb); });
+    };
+    auto cols_t = [&](int v, int nb) {
+        return brief ? time_of(8, [&] { rows_v(0, nb); cols_v(v, nb); }) : time_of(3, [&] { cols_v(v, nb); });
+    };
+    float tr[kStepVariants], tc[kStepVariants];
+    int vr = 0, vc = 0;
     // two rounds over the variants, each keeping its faster one: clocks and power settle during the
     // first, and one disturbed measurement decides nothing
     for (int round = 0; round < 2; round++)
-        for (int v = 0; v < NV; v++) {
-            const float r = rows_t(v, nprobe), c = cols_t(v, nprobe);
-            tr[v] = round ? std::min(tr[v], r) : r;
-            tc[v] = round ? std::min(tc[v], c) : c;
+        for (int v = 0; v < kStepVariants; v++) {
+            if (rows_step_has_variant(ny, v, nprobe, one_trans)) {
+                const float t = rows_t(v, nprobe);
+                tr[v] = round ? std::min(tr[v], t) : t;
+                if (round && tr[v] < tr[vr]) vr = v;
+            }
+            if (cols_step_has_variant(nx, v)) {
+                const float t = cols_t(v, nprobe);
+                tc[v] = round ? std::min(tc[v], t) : t;
+                if (round && tc[v] < tc[vc]) vc = v;
+            }
         }
-    int vr = 0, vc = 0;
-    for (int v = 1; v < NV; v++) {
-        if (tr[v] < tr[vr]) vr = v;
-        if (tc[v] < tc[vc]) vc = v;
-    }
     Tuning t{(vr ? 1 : 0) | (vc ? 2 : 0), (vr > 1 ? vr - 1 : 0) | ((vc > 1 ? vc - 1 : 0) << 2), nprobe};
-    if (m_.is_scanning() && nprobe >= 16 && (nprobe / 2) % 8 == 0) {
+    if (!brief && m_.is_scanning() && nprobe >= 16 && (nprobe / 2) % 8 == 0) {
         const float full = tr[vr] + tc[vc];
         const float half = rows_t(vr, nprobe / 2) + cols_t(vc, nprobe / 2);
         if (2.0f * half < 0.99f * full) t.nprobe = nprobe / 2;
@@ -1114,23 +1128,21 @@ Engine::Tuning Engine::tune_passes(int nprobe, ConfData& cd) {
 
 void Engine::tune(ConfData& cd) {
     const int nprobe = m_.is_scanning() ? std::min(batch_, m_.n_scan()) : ew_batch_;
-    // passes over at most 8 MB of waves (a few microseconds) are not timed: the start-up that tells the
-    // variants apart there is lost in the launches' own jitter, and per-thread loads have least of it
-    // (columns of 8 waves of 256^2: 4.4 us, bulk-copy fed 5.6 us)
-    if ((size_t)nprobe * m_.grid.nx * m_.grid.ny <= ((size_t)1 << 20)) {
-        pipe_ = shape_ = 0;
-        run_batch_ = m_.is_scanning() ? nprobe : batch_;
-        return;
-    }
     const Tuning t = tune_passes(nprobe, cd);
     pipe_ = t.pipe;
     shape_ = t.shape;
     run_batch_ = m_.is_scanning() ? std::max(1, std::min(t.nprobe, batch_)) : batch_;
 }
 
+// What the passes of the slice step run as: a pinned variant that the lengths do not have runs as the default
+// shape or with per-thread loads.
 void Engine::tuning(int* rows_variant, int* cols_variant, int* probes_per_launch) const {
-    *rows_variant = (pipe_ & 1) ? 1 + (shape_ & 3) : 0;
-    *cols_variant = (pipe_ & 2) ? 1 + ((shape_ >> 2) & 3) : 0;
+    const int nprobe = m_.is_scanning() ? run_batch_ : ew_batch_;
+    auto has_r = [&](int v) { return rows_step_has_variant(m_.grid.ny, v, nprobe, shared_trans()); };
+    auto has_c = [&](int v) { return cols_step_has_variant(m_.grid.nx, v); };
+    const int r = (pipe_ & 1) ? 1 + (shape_ & 3) : 0, c = (pipe_ & 2) ? 1 + ((shape_ >> 2) & 3) : 0;
+    *rows_variant = has_r(r) ? r : has_r(1) ? 1 : 0;
+    *cols_variant = has_c(c) ? c : has_c(1) ? 1 : 0;
     *probes_per_launch = run_batch_;
 }
 

@@ -241,6 +241,8 @@ class Engine {
     struct Tuning {
         int pipe, shape, nprobe;
     };
+    // whether every wave of a pass takes the same transmission functions (no batch of configurations)
+    bool shared_trans() const { return m_.is_scanning() || ew_batch_ == 1; }
     Tuning tune_passes(int nprobe, ConfData& cd);
     void tune(ConfData& cd);         // tune_passes for this engine's shape; sets pipe_, shape_, run_batch_
     void run_stem(ConfData& cd);

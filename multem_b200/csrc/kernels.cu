@@ -342,6 +342,37 @@ void rows_dispatch_mode(RowMode mode, const RowArgs& a, int grid_ctas, cudaStrea
 template <int NX>
 void cols_dispatch_flags(int flags, const ColArgs& a, int grid_ctas, cudaStream_t s);
 
+template <int NY>
+bool rows_has_variant(int v, int nprobe, bool one_trans);
+template <int NX>
+bool cols_has_variant(int v);
+
+bool rows_step_has_variant(int ny, int v, int nprobe, bool one_trans) {
+    switch (ny) {
+        case 64: return rows_has_variant<64>(v, nprobe, one_trans);
+        case 128: return rows_has_variant<128>(v, nprobe, one_trans);
+        case 256: return rows_has_variant<256>(v, nprobe, one_trans);
+        case 384: return rows_has_variant<384>(v, nprobe, one_trans);
+        case 512: return rows_has_variant<512>(v, nprobe, one_trans);
+        case 1024: return rows_has_variant<1024>(v, nprobe, one_trans);
+        case 2048: return rows_has_variant<2048>(v, nprobe, one_trans);
+        default: return v == 0;
+    }
+}
+
+bool cols_step_has_variant(int nx, int v) {
+    switch (nx) {
+        case 64: return cols_has_variant<64>(v);
+        case 128: return cols_has_variant<128>(v);
+        case 256: return cols_has_variant<256>(v);
+        case 384: return cols_has_variant<384>(v);
+        case 512: return cols_has_variant<512>(v);
+        case 1024: return cols_has_variant<1024>(v);
+        case 2048: return cols_has_variant<2048>(v);
+        default: return v == 0;
+    }
+}
+
 template <int N>
 constexpr int lines_per_cta() {
     return LinePlan<N>::T / (N / LinePlan<N>::E);

@@ -109,6 +109,12 @@ struct ColArgs {
     int shape;                 // pipeline shape of the bulk-copy-fed step pass (0 default, 1 or 2 an alternative where there is one)
 };
 void launch_cols(int nx, int flags, const ColArgs& a, int grid_ctas, cudaStream_t s);
+
+// Whether the slice step of this line length has the variant: 0 per-thread loads, 1 + s bulk-copy fed in
+// pipeline shape s (rows: for this many waves per launch, with one set of transmission rows for all of them or not).
+constexpr int kStepVariants = 4;
+bool rows_step_has_variant(int ny, int v, int nprobe, bool one_trans);
+bool cols_step_has_variant(int nx, int v);
 int col_det_width(int nx);      // columns per detector partial
 int col_tiles(int nx, int ny);  // detector partials per probe per detector (ny / col_det_width)
 

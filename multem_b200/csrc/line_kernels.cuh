@@ -852,6 +852,32 @@ static int max_ctas(K kernel, int threads, size_t smem) {
     return nsm * occ;
 }
 
+// Variants of the passes of the slice step: 0 per-thread loads, 1 + V bulk-copy fed in pipeline shape V, for the
+// lengths that have that shape. The dispatch below launches these, and the autotuner times no others.
+template <int NY, int V>
+constexpr bool rows_has_shape() {
+    if constexpr (V == 0 || (V == 2 && (NY == 256 || NY == 2048)))
+        return RowPipe<NY, RowPipeShape<NY, V>::GT, RowPipeShape<NY, V>::NG, RowPipeShape<NY, V>::PM>::OK;
+    else return false;
+}
+template <int NX, int V>
+constexpr bool cols_has_shape() {
+    if constexpr (V == 0 || (V == 1 && (NX == 256 || NX == 512)) || (V == 2 && (NX == 384 || NX == 1024)))
+        return ColPipe<NX, ColPipeShape<NX, V>::GT, ColPipeShape<NX, V>::NG, ColPipeShape<NX, V>::PM, ColPipeShape<NX, V>::OWN>::OK;
+    else return false;
+}
+// The bulk-copy-fed rows share the resident transmission rows over the batch and take whole groups of waves.
+template <int NY>
+bool rows_has_variant(int v, int nprobe, bool one_trans) {
+    return v == 0 || (one_trans && ((v == 1 && rows_has_shape<NY, 0>() && nprobe % RowPipeShape<NY, 0>::NG == 0) ||
+                                    (v == 3 && rows_has_shape<NY, 2>() && nprobe % RowPipeShape<NY, 2>::NG == 0)));
+}
+template <int NX>
+bool cols_has_variant(int v) {
+    return v == 0 || (v == 1 && cols_has_shape<NX, 0>()) || (v == 2 && cols_has_shape<NX, 1>()) ||
+           (v == 3 && cols_has_shape<NX, 2>());
+}
+
 // Launches the bulk-copy-fed row pass in pipeline shape V when that shape fits this line length and
 // the probe count; returns false otherwise.
 template <int NY, int MODE, int V>
@@ -882,7 +908,7 @@ template <int NY, int MODE>
 static void rows_launch(const RowArgs& a, int grid_ctas, cudaStream_t s) {
     using G = LineGeom<NY>;
     if (a.err) {
-        if constexpr (MODE == ROW_STEP && (NY == 256 || NY == 2048))
+        if constexpr (MODE == ROW_STEP && rows_has_shape<NY, 2>())
             if (a.shape == 2 && rows_pipe_try<NY, MODE, 2>(a, grid_ctas, s)) return;
         if (rows_pipe_try<NY, MODE, 0>(a, grid_ctas, s)) return;
     }
@@ -936,9 +962,9 @@ static void cols_launch_ld(const ColArgs& a, int grid_ctas, cudaStream_t s) {
     using G = LineGeom<NX>;
     if (a.err) {
         if constexpr (FLAGS == (COL_LOAD | COL_PROP | COL_INVERSE | COL_STORE)) {
-            if constexpr (ColPipeShape<NX, 1>::OWN)
+            if constexpr (cols_has_shape<NX, 1>())
                 if (a.shape == 1 && cols_pipe_try<NX, FLAGS, LDY, 1>(a, grid_ctas, s)) return;
-            if constexpr (NX == 384 || NX == 1024)
+            if constexpr (cols_has_shape<NX, 2>())
                 if (a.shape == 2 && cols_pipe_try<NX, FLAGS, LDY, 2>(a, grid_ctas, s)) return;
         }
         if (cols_pipe_try<NX, FLAGS, LDY, 0>(a, grid_ctas, s)) return;

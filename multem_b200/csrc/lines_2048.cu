@@ -5,4 +5,6 @@ namespace mtb {
 template void rows_dispatch_mode<2048>(RowMode, const RowArgs&, int, cudaStream_t);
 template void cols_dispatch_flags<2048>(int, const ColArgs&, int, cudaStream_t);
 template int cols_det_width<2048>();
+template bool rows_has_variant<2048>(int, int, bool);
+template bool cols_has_variant<2048>(int);
 }  // namespace mtb

@@ -85,3 +85,38 @@ def test_autotuner_reports_its_choice():
     e.close()
     assert t["rows"] in (0, 1, 2, 3) and t["cols"] in (0, 1, 2, 3)
     assert t["probes_per_launch"] in (128, 256)
+
+
+ROWS = {64: (0, 1), 128: (0, 1), 256: (0, 1, 3), 384: (0, 1), 512: (0, 1), 1024: (0, 1), 2048: (0, 1, 3)}
+COLS = {64: (0, 1), 128: (0, 1), 256: (0, 1, 2), 384: (0, 1, 3), 512: (0, 1, 2), 1024: (0, 1, 3), 2048: (0, 1)}
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 2048), (128, 64), (256, 1024), (384, 512), (512, 256), (1024, 384), (2048, 128)])
+def test_only_variants_of_the_lengths_are_reported(nx, ny, monkeypatch):
+    """The autotuner chooses, and mt_engine_tuning reports, variants that the line lengths have; one wave, or several with
+    transmission functions of their own, have no bulk-copy-fed rows."""
+    p = specimens.hrtem_si001(nx=nx, ny=ny, na=2, nb=2, nc=2)
+    q = specimens.stem_srtio3(nx=nx, ny=ny, na=4, nb=4, nc=2, ns=4, nconf=1, seed=3)
+    for spec, rows in ((p, (0,)), (q, ROWS[ny])):
+        for pin in (None, "0", "5", "10"):
+            if pin is None:
+                monkeypatch.delenv("MTB_PIPE", raising=False)
+            else:
+                monkeypatch.setenv("MTB_PIPE", "3")
+                monkeypatch.setenv("MTB_SHAPE", pin)
+            e = api.Engine(spec)
+            e.run()
+            t = e.tuning()
+            e.close()
+            assert t["rows"] in rows and t["cols"] in COLS[nx], (pin, t)
+
+
+def test_short_passes_are_tuned_too():
+    """Columns of 1024 points are faster bulk-copy fed however few they are (1024 x 128, one wave: 17 us a slice
+    with per-thread loads, 13 us)."""
+    p = specimens.hrtem_si001(nx=1024, ny=128, na=2, nb=2, nc=4)
+    e = api.Engine(p)
+    e.run()
+    t = e.tuning()
+    e.close()
+    assert t["cols"] in (1, 3)
