@@ -214,7 +214,7 @@ __device__ __forceinline__ void gather_items(const Source& src, const long long 
 }
 
 // Planes dst[p][s] (p < nplane, s < npix) of the channels c0 .. c0 + 8*nplane - 1 at the pixel offsets
-// s_off, by all threads; use(v) sees every piece.
+// s_off, by all threads; use(v, p) sees every piece.
 template <bool FULL, bool MASK, class Use>
 __device__ __forceinline__ void gather_planes(const Source& src, const long long* s_off, int c0, int nplane, int npix,
                                               uint4* dst, Use use) {
@@ -237,7 +237,7 @@ __device__ __forceinline__ void gather_planes(const Source& src, const long long
         for (int u = 0; u < U; u++) {
             const int at = e + u * THREADS;
             if (at < nplane * npix) dst[at] = v[u];
-            use(v[u]);
+            use(v[u], (c[u] - c0) / 8);
         }
     }
 }
@@ -290,9 +290,9 @@ __device__ __forceinline__ void weights8(const __nv_bfloat16* w, int row, int nr
     }
 }
 
-// whether either bf16 of a word is an infinity or NaN (exponent bits all set)
-__device__ __forceinline__ int nonfinite(uint32_t u) {
-    return (u & 0x7F80u) == 0x7F80u || (u & 0x7F800000u) == 0x7F800000u;
+// whether the low (bit 0) and the high (bit 1) bf16 of a word are infinities or NaN (exponent bits all set)
+__device__ __forceinline__ unsigned nonfinite(uint32_t u) {
+    return ((u & 0x7F80u) == 0x7F80u ? 1u : 0u) | ((u & 0x7F800000u) == 0x7F800000u ? 2u : 0u);
 }
 
 struct ConvArgs {
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
                 for (int t = 0; t < 9; t++) wt[((8 - t) * (BN / 8) + p) * kw + k] = v[t];
             }
         }
-        gather({in, mask, hw, a.Cin}, s_off, (kb0 + kb) * kw, nplane, npix, reinterpret_cast<uint4*>(st), [](uint4) {});
+        gather({in, mask, hw, a.Cin}, s_off, (kb0 + kb) * kw, nplane, npix, reinterpret_cast<uint4*>(st), [](uint4, int) {});
         fence_proxy_async();
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -549,7 +549,7 @@ struct WgradArgs {
     const __nv_bfloat16* mask;  // zero dout where not positive, or NULL
     float* part;                // [split][ky][kx][Cin][Cout32], Cout32 = Cout rounded up to WG_OC
     float* bpart;               // [split][Cout32]
-    int* special;               // [split][input tile][output tile]: the inputs hold an infinity or NaN
+    unsigned* special;          // [split][Cin / 32]: bit per input channel, whether it holds an infinity or NaN
     Image im;
     int Cin, Cout;
     int nblk, blk_per_split;    // K blocks of WG_PIX pixels, and per split
@@ -580,7 +580,7 @@ struct WgradTile {
 // are MN-major. The bias gradient is summed from the gathered values (input tile 0). FP32 partial
 // sums per split, added in split order by wgrad_finalize_kernel. The zeros between rows and images
 // take part in the products, so an infinite or NaN input beside them would reach taps that it has no
-// part in: such inputs are noted (WgradArgs::special) and their sums taken without the padding.
+// part in: such channels are noted for the split (WgradArgs::special) and their sums taken without the padding.
 // 16 images of 32 -> 32 channels at 128 x 128: 53 us and 8 us for the finalize kernel (transposed im2col,
 // GEMM and finalize through memory: 195 us).
 template <int NI>
@@ -590,6 +590,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
     __shared__ unsigned long long done[2];
     __shared__ unsigned s_tmem;
     __shared__ float s_bias[THREADS / 32][8];
+    __shared__ unsigned s_special[(NI + 31) / 32];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int W = a.im.W, Wp = W + 1;
     const size_t hw = (size_t)a.im.H * W;
@@ -599,6 +600,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
     long long* s_goff = s_off + npix;                            // gradient pixels -1 .. WG_PIX
     unsigned char* stage0 = conv_smem + 8 * (size_t)(npix + WG_PIX + 2);
     const size_t stage_bytes = T::stage_bytes(W);
+    if (threadIdx.x < (NI + 31) / 32) s_special[threadIdx.x] = 0u;
     if (threadIdx.x == 0) {
         mbar_init(&done[0], 1);
         mbar_init(&done[1], 1);
@@ -615,7 +617,6 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
     const int blk0 = blockIdx.x * a.blk_per_split;
     const int nb = a.nblk - blk0 < a.blk_per_split ? a.nblk - blk0 : a.blk_per_split;
     bool ok = !err_set(a.err);
-    int special = 0;
     float bsum[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) bsum[j] = 0.0f;
@@ -681,8 +682,10 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
             }
         }
         const __nv_bfloat16* in = a.in + (size_t)b0 * a.Cin * hw;
-        gather({in, nullptr, hw, a.Cin}, s_off, i0, NI / 8, npix, xin,
-               [&](uint4 v) { special |= nonfinite(v.x) | nonfinite(v.y) | nonfinite(v.z) | nonfinite(v.w); });
+        gather({in, nullptr, hw, a.Cin}, s_off, i0, NI / 8, npix, xin, [&](uint4 v, int p) {
+            const unsigned bits = nonfinite(v.x) | nonfinite(v.y) << 2 | nonfinite(v.z) << 4 | nonfinite(v.w) << 6;
+            if (bits) atomicOr(&s_special[p / 4], bits << 8 * (p % 4));
+        });
         fence_proxy_async();
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -716,8 +719,9 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
                 if (i + j < a.Cin) dst[(size_t)j * C32] = ok ? __uint_as_float(r[j]) : 0.0f;
         }
     }
-    special = __syncthreads_or(special);
-    if (threadIdx.x == 0) a.special[((size_t)blockIdx.x * gridDim.y + blockIdx.y) * gridDim.z + blockIdx.z] = special;
+    // the last block's barrier came after every note
+    const int words = (a.Cin + 31) / 32, w0 = i0 / 32 + threadIdx.x;
+    if (blockIdx.z == 0 && threadIdx.x < (NI + 31) / 32 && w0 < words) a.special[(size_t)blockIdx.x * words + w0] = s_special[threadIdx.x];
     if (blockIdx.y == 0) {
 #pragma unroll
         for (int j = 0; j < 8; j++)
@@ -739,12 +743,49 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
     }
 }
 
+// Adds what split k sums for output channel o (a lane's), input channel i and the three taps kx of ky: the
+// gradient's pixels q whose input column q + kx - 1 lies in the split's range. Returns true, early, once the sums
+// of every lane are NaN.
+__device__ __forceinline__ bool direct_sums(const WgradArgs& a, int i, int o, int ky, int k, float (&acc)[3]) {
+    const int H = a.im.H, W = a.im.W;
+    const long long q0 = (long long)k * a.blk_per_split * WG_PIX, q1 = q0 + (long long)a.blk_per_split * WG_PIX;
+    const long long first = q0 > 0 ? q0 - 1 : 0;
+    int b, y, x;
+    uint32_t r;
+    locate(a.im, first, b, r);
+    y = (int)(r / (uint32_t)(W + 1));
+    x = (int)(r - (uint32_t)y * (uint32_t)(W + 1));
+    for (long long q = first; q <= q1 && b < a.im.B; q++) {
+        if (y < H && x < W) {
+            const int yy = y + ky - 1;
+            const bool row = yy >= 0 && yy < H;
+            const __nv_bfloat16* xi = a.in + (((size_t)b * a.Cin + i) * H + (row ? yy : 0)) * W;
+            const size_t go = (((size_t)b * a.Cout + (o < a.Cout ? o : 0)) * H + y) * W + x;
+            float g = __bfloat162float(a.dout[go]);
+            if (a.mask && !(__bfloat162float(a.mask[go]) > 0.0f)) g = 0.0f;
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+                const int xx = x + t - 1;
+                // outside the image the input is zero (times an infinite gradient: NaN)
+                if (q + t - 1 >= q0 && q + t - 1 < q1)
+                    acc[t] = __fmaf_rn(g, row && xx >= 0 && xx < W ? __bfloat162float(xi[xx]) : 0.0f, acc[t]);
+            }
+            if (__all_sync(0xffffffffu, isnan(acc[0]) && isnan(acc[1]) && isnan(acc[2]))) return true;
+        }
+        if (++x > W) {
+            x = 0;
+            if (++y > H) y = 0, b++;
+        }
+    }
+    return false;
+}
+
 // dw[o][i][tap] and db[o] from the splits' partial sums: one CTA per (32 output channels, input
 // channel, ky); warp v adds splits v, v + 8, ... in order, then the eight warps' sums are added in
-// order. The CTA row i = Cin does the bias. With infinities or NaN in the tile's inputs the sums run
-// over the image pixels themselves (rows strided over the warps).
-__global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, int splits, int itiles, int NI,
-                                                             float* dw, float* db) {
+// order. The CTA row i = Cin does the bias. Where a split's input channel holds an infinity or NaN, the split's
+// sum runs over its image pixels themselves, until every sum of the warp is NaN, which nothing changes
+// any more.
+__global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, int splits, float* dw, float* db) {
     __shared__ float s[8][3][32];
     next_may_start();
     previous_done();
@@ -753,39 +794,33 @@ __global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, 
     const bool bias = i == a.Cin;
     if (bias && ky > 0) return;
     float acc[3] = {0.0f, 0.0f, 0.0f};
-    int special = 0;
+    const int words = (a.Cin + 31) / 32;
+    auto special = [&](int k) { return a.special[(size_t)k * words + i / 32] >> (i % 32) & 1u; };
+    unsigned any = 0;
+    const float* p = a.part + ((size_t)(3 * ky) * a.Cin + i) * C32 + o;
+    const size_t tap = (size_t)a.Cin * C32, split = 9 * tap;
     if (bias) {
         for (int k = warp; k < splits; k += 8) acc[0] += a.bpart[(size_t)k * C32 + o];
     } else {
-        for (int k = threadIdx.x; k < splits; k += 256)
-            special |= a.special[((size_t)k * itiles + i / NI) * gridDim.x + blockIdx.x];
-        const float* p = a.part + ((size_t)(3 * ky) * a.Cin + i) * C32 + o;
-        const size_t tap = (size_t)a.Cin * C32, split = 9 * tap;
+        for (int k = threadIdx.x; k < splits; k += 256) any |= special(k);
 #pragma unroll 4
         for (int k = warp; k < splits; k += 8)
 #pragma unroll
             for (int t = 0; t < 3; t++) acc[t] += p[k * split + t * tap];
     }
-    if (__syncthreads_or(special)) {
-        const int H = a.im.H, W = a.im.W;
+    if (__syncthreads_or((int)any)) {
+        float sum[3] = {0.0f, 0.0f, 0.0f};
+        bool nan = false;
+        for (int k = warp; k < splits && !nan; k += 8) {
+            if (special(k)) {
+                nan = direct_sums(a, i, o, ky, k, sum);
+            } else {
 #pragma unroll
-        for (int t = 0; t < 3; t++) acc[t] = 0.0f;
-        for (int by = warp; o < a.Cout && by < a.im.B * H; by += 8) {
-            const int b = by / H, y = by - b * H, yy = y + ky - 1;
-            const bool row = yy >= 0 && yy < H;
-            const __nv_bfloat16* xi = a.in + (((size_t)b * a.Cin + i) * H + (row ? yy : 0)) * W;
-            const size_t go = (((size_t)b * a.Cout + o) * H + y) * W;
-            for (int x = 0; x < W; x++) {
-                float g = __bfloat162float(a.dout[go + x]);
-                if (a.mask && !(__bfloat162float(a.mask[go + x]) > 0.0f)) g = 0.0f;
-#pragma unroll
-                for (int t = 0; t < 3; t++) {
-                    const int xx = x + t - 1;
-                    // outside the image the input is zero (times an infinite gradient: NaN)
-                    acc[t] = __fmaf_rn(g, row && xx >= 0 && xx < W ? __bfloat162float(xi[xx]) : 0.0f, acc[t]);
-                }
+                for (int t = 0; t < 3; t++) sum[t] += p[k * split + t * tap];
             }
         }
+#pragma unroll
+        for (int t = 0; t < 3; t++) acc[t] = sum[t];
     }
 #pragma unroll
     for (int t = 0; t < 3; t++) s[warp][t][lane] = acc[t];

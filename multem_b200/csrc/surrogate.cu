@@ -241,17 +241,17 @@ void wgrad_launch(mtb::conv::WgradArgs a, float* dw, float* db, cudaStream_t st)
     const int splits = (a.nblk + a.blk_per_split - 1) / a.blk_per_split;
     const size_t off_b = align256((size_t)splits * 9 * a.Cin * C32 * sizeof(float));
     const size_t off_s = off_b + align256((size_t)splits * C32 * sizeof(float));
-    Workspace& ws = workspace(off_s + (size_t)splits * itiles * otiles * sizeof(int));
+    Workspace& ws = workspace(off_s + (size_t)splits * ((a.Cin + 31) / 32) * sizeof(unsigned));
     a.part = reinterpret_cast<float*>(ws.p);
     a.bpart = reinterpret_cast<float*>(ws.p + off_b);
-    a.special = reinterpret_cast<int*>(ws.p + off_s);
+    a.special = reinterpret_cast<unsigned*>(ws.p + off_s);
     a.err = ws.err;
     auto kern = mtb::conv::wgrad_kernel<NI>;
     const size_t smem = T::smem(a.im.W);
     MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     mtb::launch_early(true, kern, dim3((unsigned)splits, (unsigned)itiles, (unsigned)otiles), mtb::conv::THREADS, smem, st, a);
     mtb::launch_early(true, mtb::conv::wgrad_finalize_kernel, dim3((unsigned)otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st, a, splits,
-                      itiles, NI, dw, db);
+                      dw, db);
 }
 
 }  // namespace
