@@ -797,12 +797,18 @@ __global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, 
     const int words = (a.Cin + 31) / 32;
     auto special = [&](int k) { return a.special[(size_t)k * words + i / 32] >> (i % 32) & 1u; };
     unsigned any = 0;
+    float first = 0.0f;
     const float* p = a.part + ((size_t)(3 * ky) * a.Cin + i) * C32 + o;
     const size_t tap = (size_t)a.Cin * C32, split = 9 * tap;
     if (bias) {
         for (int k = warp; k < splits; k += 8) acc[0] += a.bpart[(size_t)k * C32 + o];
     } else {
         for (int k = threadIdx.x; k < splits; k += 256) any |= special(k);
+        // the line's first pixel meets the zero before it in no split: nothing, or NaN for an infinite gradient
+        if (warp == 0 && o < a.Cout) {
+            const size_t go = (size_t)o * a.im.H * a.im.W;
+            if (!a.mask || __bfloat162float(a.mask[go]) > 0.0f) first = __bfloat162float(a.dout[go]) * 0.0f;
+        }
 #pragma unroll 4
         for (int k = warp; k < splits; k += 8)
 #pragma unroll
@@ -822,6 +828,7 @@ __global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, 
 #pragma unroll
         for (int t = 0; t < 3; t++) acc[t] = sum[t];
     }
+    acc[0] += first;
 #pragma unroll
     for (int t = 0; t < 3; t++) s[warp][t][lane] = acc[t];
     __syncthreads();

@@ -94,6 +94,30 @@ def test_weight_gradient_with_infinite_and_nan_inputs():
     assert _rel(dw[ok], ref[ok]) < 1e-4
 
 
+@pytest.mark.parametrize("at", [(0, 0, 0), (0, 0, 5), (0, 4, 0), (1, 0, 0), (1, 4, 5), (1, 2, 3)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_weight_gradient_with_an_infinite_gradient(value, at):
+    """An infinite gradient times the zero beside the image is NaN, at the corners of the first and the last image too."""
+    torch = pytest.importorskip("torch")
+    lib = capi.load()
+    B, Cin, Cout, H, W = 2, 3, 4, 5, 6
+    g = torch.Generator().manual_seed(9)
+    x = (1 + torch.rand(B, Cin, H, W, generator=g)).to(torch.bfloat16)
+    d = torch.randn(B, Cout, H, W, generator=g)
+    d[at[0], 2, at[1], at[2]] = value
+    d = d.to(torch.bfloat16)
+    cols = torch.nn.functional.unfold(x.double(), 3, padding=1).reshape(B, Cin, 9, H * W)
+    ref = torch.einsum("boq,bctq->oct", d.double().reshape(B, Cout, H * W), cols).reshape(Cout, Cin, 3, 3)
+    xd, dd = x.cuda(), d.cuda()
+    dw, db = torch.empty(Cout, Cin, 3, 3, device="cuda"), torch.empty(Cout, device="cuda")
+    capi.check(lib.mt_sg_conv3x3_backward_weight(_p(xd), _p(dd), None, _p(dw), _p(db), B, Cin, Cout, H, W, None))
+    dw, db = dw.cpu().double(), db.cpu()
+    assert torch.equal(dw.isnan(), ref.isnan()) and torch.equal(dw.isinf(), ref.isinf())
+    ok = ref.isfinite()
+    assert _rel(dw[ok], ref[ok]) < 1e-4
+    assert torch.equal(db.isfinite(), torch.tensor([True, True, False, True]))
+
+
 # infinities and NaN in some channels and splits of a layer of many (296 splits of 8 blocks), and everywhere
 @pytest.mark.parametrize("what", ["few", "one channel", "all"])
 def test_weight_gradient_with_infinite_and_nan_inputs_of_a_large_layer(what):
