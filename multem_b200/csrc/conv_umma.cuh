@@ -81,15 +81,18 @@ __device__ __forceinline__ void mma_commit(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
+// The load and its wait are one statement: nothing ties the registers to a wait of its own, so arithmetic on them
+// could be placed before it.
 __device__ __forceinline__ void tmem_ld16(unsigned taddr, uint32_t (&r)[16]) {  // whole warp
     __syncwarp();  // the instruction needs the warp together, whatever branches came before
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15}, [%16];"
+        "%15}, [%16];\n"
+        " tcgen05.wait::ld.sync.aligned;"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        : "r"(taddr)
+        : "memory");
 }
 
 // Barrier over the threads of the cluster's CTAs, ordering their shared memory. Not the .aligned form: a warp's

@@ -43,6 +43,17 @@ def test_kernels_that_start_early_use_ordinary_loads():
             assert not re.search(r"__ldg|ld\.global\.nc|const\s+\w+\*\s*__restrict__\s+\w+\s*=", src), f"{file}: non-coherent load"
 
 
+def test_tensor_memory_loads_wait_in_the_same_statement():
+    """Registers of a tensor-memory load are undefined until its wait, and only one asm statement keeps their use behind it."""
+    loads = 0
+    for file, src in _sources().items():
+        for m in re.finditer(r"asm\b[^;]*?\((?:[^()\"]|\"[^\"]*\"|\((?:[^()]|\([^()]*\))*\))*\)\s*;", src):
+            if "tcgen05.ld" in m.group(0):
+                loads += 1
+                assert "tcgen05.wait::ld" in m.group(0), file
+    assert loads >= 1
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,ch,H,W", [(1, 16, 16, 16), (2, 40, 33, 17), (8, 32, 64, 64), (4, 256, 8, 8)])
 def test_chain_over_alternating_buffers_equals_waited_calls(B, ch, H, W):
