@@ -392,9 +392,9 @@ __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
     }
     tc_fence_before();
     __syncthreads();
-    // only now, so that no CTA of a later kernel can hold tensor memory that one of this kernel waits for
-    next_may_start();
     previous_done();
+    // not before the allocation: no CTA of a later kernel may hold tensor memory that one of this kernel waits for
+    next_may_start();
     const __nv_bfloat16* in = a.in + (size_t)b0 * a.Cin * hw;
     const __nv_bfloat16* mask = a.mask ? a.mask + (size_t)b0 * a.Cin * hw : nullptr;
 
@@ -614,8 +614,8 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = s_tmem;
-    next_may_start();  // after the allocation, as in conv_kernel
     previous_done();
+    next_may_start();  // after the allocation, as in conv_kernel
 
     const int blk0 = blockIdx.x * a.blk_per_split;
     const int nb = a.nblk - blk0 < a.blk_per_split ? a.nblk - blk0 : a.blk_per_split;
@@ -790,8 +790,8 @@ __device__ __forceinline__ bool direct_sums(const WgradArgs& a, int i, int o, in
 // any more.
 __global__ void __launch_bounds__(256) wgrad_finalize_kernel(const WgradArgs a, int splits, float* dw, float* db) {
     __shared__ float s[8][3][32];
-    next_may_start();
     previous_done();
+    next_may_start();
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int o = blockIdx.x * 32 + lane, i = blockIdx.y, ky = blockIdx.z, C32 = gridDim.x * 32;
     const bool bias = i == a.Cin;

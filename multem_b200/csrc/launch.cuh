@@ -4,7 +4,10 @@
 // layout), and must call previous_done() before it reads or writes any memory that an earlier kernel
 // touches. A kernel that calls next_may_start() lets its successor start once every CTA has called it; a
 // kernel that calls neither behaves as ever. Since every early kernel waits for its predecessor's end
-// before its own, the order holds along the whole stream.
+// before its own, the order holds along the whole stream. next_may_start() comes after previous_done(): a kernel's
+// successor then starts when the kernel's predecessor has ended, and no more than two are resident. Called first,
+// a third could be, whose SM may still load, for the first, the old contents of a buffer that the second writes and
+// it reads itself.
 //
 // What an early kernel reads may be written while it is resident, so it is read with ordinary loads only:
 // no __ldg, which wants memory that nothing writes for as long as the kernel runs, and no __restrict__, which

@@ -39,8 +39,8 @@ __global__ void surrogate_loss_kernel(const float* head, const __nv_bfloat16* x,
                                       const float* t, const float* scale,
                                       __nv_bfloat16* dhead, float* terms, int B, int HW,
                                       float lambda) {
-    mtb::next_may_start();
     mtb::previous_done();
+    mtb::next_may_start();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= B * HW) return;
     const int b = p / HW, q = p % HW;
@@ -59,8 +59,8 @@ __global__ void surrogate_loss_kernel(const float* head, const __nv_bfloat16* x,
 __global__ void adam_kernel(float* wm, __nv_bfloat16* wb, const float* g,
                             float* m, float* v, int n, float lr, float b1, float b2, float eps,
                             float c1, float c2) {
-    mtb::next_may_start();
     mtb::previous_done();
+    mtb::next_may_start();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -77,8 +77,8 @@ __global__ void adam_kernel(float* wm, __nv_bfloat16* wb, const float* g,
 // the gradient of nearest-neighbour upsampling with scale 1.
 __global__ void pool2_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, int planes, int H,
                              int W, float scale) {
-    mtb::next_may_start();
     mtb::previous_done();
+    mtb::next_may_start();
     const int Ho = H / 2, Wo = W / 2;
     const size_t n = (size_t)planes * Ho * Wo;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -94,8 +94,8 @@ __global__ void pool2_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, int pl
 // scale 1, the gradient of average pooling with scale 1/4.
 __global__ void upsample2_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, int planes,
                                  int H, int W, float scale) {
-    mtb::next_may_start();
     mtb::previous_done();
+    mtb::next_may_start();
     const int Ho = 2 * H, Wo = 2 * W;
     const size_t n = (size_t)planes * Ho * Wo;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -107,8 +107,8 @@ __global__ void upsample2_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, in
 
 __global__ void add_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b,
                            __nv_bfloat16* out, size_t n) {
-    mtb::next_may_start();
     mtb::previous_done();
+    mtb::next_may_start();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         out[k] = __float2bfloat16_rn(bf(a[k]) + bf(b[k]));
 }

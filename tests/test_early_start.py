@@ -18,7 +18,7 @@ def _sources():
 
 
 def _early_kernels():
-    """(file, name, parameters) of every kernel whose body waits for its predecessor itself."""
+    """(file, name, parameters, body) of every kernel whose body waits for its predecessor itself."""
     found = []
     for name, src in _sources().items():
         for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(([^)]*)\)\s*\{", src):
@@ -27,20 +27,27 @@ def _early_kernels():
                 depth += {"{": 1, "}": -1}.get(src[i], 0)
                 i += 1
             if "previous_done()" in src[m.end():i]:
-                found.append((name, m.group(1), m.group(2)))
+                found.append((name, m.group(1), m.group(2), src[m.end():i]))
     return found
 
 
 def test_kernels_that_start_early_use_ordinary_loads():
     early = _early_kernels()
-    names = {k for _, k, _ in early}
+    names = {k for _, k, _, _ in early}
     assert {"rows_kernel", "rows_pipe_kernel", "cols_kernel", "cols_pipe_kernel", "splat_kernel", "det_reduce_kernel",
             "ew_accumulate_kernel", "conv_kernel", "wgrad_kernel", "wgrad_finalize_kernel", "adam_kernel"} <= names
-    for file, kernel, params in early:
+    for file, kernel, params, _ in early:
         assert "__restrict__" not in params, f"{file}: {kernel} has __restrict__ parameters"
     for file, src in _sources().items():
-        if file in {f for f, _, _ in early} | {"fft_core.cuh", "mbarrier.cuh"}:
+        if file in {f for f, _, _, _ in early} | {"fft_core.cuh", "mbarrier.cuh"}:
             assert not re.search(r"__ldg|ld\.global\.nc|const\s+\w+\*\s*__restrict__\s+\w+\s*=", src), f"{file}: non-coherent load"
+
+
+def test_successors_start_after_the_wait():
+    """No kernel lets its successor start before it has waited for its predecessor: two are resident, never three."""
+    for file, kernel, _, body in _early_kernels():
+        if "next_may_start()" in body:
+            assert body.index("previous_done()") < body.index("next_may_start()"), f"{file}: {kernel}"
 
 
 def test_tensor_memory_loads_wait_in_the_same_statement():
