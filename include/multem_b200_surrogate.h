@@ -31,6 +31,11 @@ mt_status mt_sg_conv3x3_backward_data(const void* dout, const void* out_mask, co
  * above). */
 mt_status mt_sg_conv3x3_backward_weight(const void* in, const void* dout, const void* out_mask, float* dw, float* db,
                                         int B, int Cin, int Cout, int H, int W, void* stream);
+/* How such a layer is cut (host only; pass 0 forward, 1 data gradient, 2 weight gradient), plan[5]: channels per
+ * CTA (output channels; input channels for the weight gradient), pixel tiles of 128 per CTA, CTAs that share the sum
+ * (over input channels; over pixels for the weight gradient), blocks of it per CTA, and whether the pixels
+ * around a tile are gathered as three segments (wide rows) instead of one band. */
+mt_status mt_sg_conv3x3_plan(int B, int Cin, int Cout, int H, int W, int pass, int* plan);
 /* Loss of the two-channel head (float [B,2,H,W]) in units of a per-item scale s_b (float [B], or
  * NULL for 1): channel 0 corrects the input image x (bf16 [B,1,H,W]) towards target (float
  * [B,1,H,W]) as x + s_b * head0, channel 1 estimates |x + s_b * head0 - target| / s_b. Per pixel

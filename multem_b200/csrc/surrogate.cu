@@ -202,46 +202,70 @@ void conv_launch(const mtb::conv::ConvArgs& a, cudaStream_t st) {
     MTB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
 }
 
-// The widest tile (up to 64 output channels: more would leave room for one CTA per SM only) that, with
-// the input channels shared over up to 8 CTAs, still gives every SM a CTA; two pixel tiles per CTA
-// where there are CTAs to spare.
-template <bool DGRAD>
-void conv(mtb::conv::ConvArgs a, cudaStream_t st) {
-    const long long tiles = (a.im.total() + 127) / 128;
-    const int nkb = (a.Cin + mtb::conv::KC - 1) / mtb::conv::KC;
+// How a convolution is cut. The widest tile (up to 64 output channels: more would leave room for one CTA per SM
+// only) that, with the input channels shared over up to 8 CTAs, still gives every SM a CTA; two pixel tiles per
+// CTA where there are CTAs to spare.
+struct ConvPlan {
+    int bn, ksplit, blocks;  // output channels per CTA, CTAs that share the input channels, K blocks of each
+    bool two;                // pixel tiles per CTA
+};
+ConvPlan conv_plan(const mtb::conv::Image& im, int Cin, int Cout) {
+    const long long tiles = (im.total() + 127) / 128;
+    const int nkb = (Cin + mtb::conv::KC - 1) / mtb::conv::KC;
     int most = 1;
     while (most < 8 && 2 * most <= nkb) most *= 2;
-    auto ctas = [&](int bn) { return tiles * ((a.Cout + bn - 1) / bn); };
-    int bn = a.Cout <= 16 ? 16 : a.Cout <= 32 ? 32 : 64;
-    while (bn > 16 && ctas(bn) * most < 148) bn /= 2;
+    auto ctas = [&](int bn) { return tiles * ((Cout + bn - 1) / bn); };
+    ConvPlan p{Cout <= 16 ? 16 : Cout <= 32 ? 32 : 64, 1, nkb, false};
+    while (p.bn > 16 && ctas(p.bn) * most < 148) p.bn /= 2;
     // K is cut into `parts` at least (over CTAs and accumulators) where that leaves more than two blocks to each CTA
-    const long long m = ((long long)a.im.B * a.im.H * a.im.W + 127) / 128 * ((a.Cout + 255) / 256);
+    const long long m = ((long long)im.B * im.H * im.W + 127) / 128 * ((Cout + 255) / 256);
     const long long parts = (295 + m) / m;
-    a.ksplit = 1;
-    while (a.ksplit < most && (ctas(bn) * a.ksplit < 148 ||
-                               (nkb + a.ksplit - 1) / a.ksplit > std::max<long long>(2, 4 * nkb / parts)))
-        a.ksplit *= 2;
-    const bool two = ctas(bn) >= 4 * 148 && parts == 1;
-    switch (bn) {
-        case 16: two ? conv_launch<16, 2, DGRAD>(a, st) : conv_launch<16, 1, DGRAD>(a, st); break;
-        case 32: two ? conv_launch<32, 2, DGRAD>(a, st) : conv_launch<32, 1, DGRAD>(a, st); break;
-        default: two ? conv_launch<64, 2, DGRAD>(a, st) : conv_launch<64, 1, DGRAD>(a, st); break;
+    while (p.ksplit < most && (ctas(p.bn) * p.ksplit < 148 || p.blocks > std::max<long long>(2, 4 * nkb / parts))) {
+        p.ksplit *= 2;
+        p.blocks = (nkb + p.ksplit - 1) / p.ksplit;
+    }
+    p.two = ctas(p.bn) >= 4 * 148 && parts == 1;
+    return p;
+}
+
+template <bool DGRAD>
+void conv(mtb::conv::ConvArgs a, cudaStream_t st) {
+    const ConvPlan p = conv_plan(a.im, a.Cin, a.Cout);
+    a.ksplit = p.ksplit;
+    switch (p.bn) {
+        case 16: p.two ? conv_launch<16, 2, DGRAD>(a, st) : conv_launch<16, 1, DGRAD>(a, st); break;
+        case 32: p.two ? conv_launch<32, 2, DGRAD>(a, st) : conv_launch<32, 1, DGRAD>(a, st); break;
+        default: p.two ? conv_launch<64, 2, DGRAD>(a, st) : conv_launch<64, 1, DGRAD>(a, st); break;
     }
 }
 
+// How a weight gradient is cut: input channels per CTA (the gradient tile is gathered once for each, so as many as
+// the layer has and two stages of shared memory hold) and K blocks per split, for two CTAs per SM (one
+// where the tile's tensor memory allows no more).
+struct WgradPlan {
+    int ni, itiles, otiles, nblk, blk_per_split, splits;
+};
+WgradPlan wgrad_plan(const mtb::conv::Image& im, int Cin, int Cout) {
+    WgradPlan p{};
+    p.ni = Cin <= 16 ? 16 : Cin <= 32 ? 32 : Cin <= 64 || mtb::conv::WgradTile<128>::smem(im.W) > (size_t)kSmemMax ? 64 : 128;
+    p.itiles = (Cin + p.ni - 1) / p.ni;
+    p.otiles = (Cout + mtb::conv::WG_OC - 1) / mtb::conv::WG_OC;
+    p.nblk = (int)((im.total() + mtb::conv::WG_PIX - 1) / mtb::conv::WG_PIX);
+    const long long tiles = (long long)p.itiles * p.otiles, want = ((p.ni > 64 ? 148 : 296) + tiles - 1) / tiles;
+    p.blk_per_split = (int)std::max<long long>(1, (p.nblk + want - 1) / want);
+    p.splits = (p.nblk + p.blk_per_split - 1) / p.blk_per_split;
+    return p;
+}
+
 template <int NI>
-void wgrad_launch(mtb::conv::WgradArgs a, float* dw, float* db, cudaStream_t st) {
+void wgrad_launch(mtb::conv::WgradArgs a, const WgradPlan& p, float* dw, float* db, cudaStream_t st) {
     using T = mtb::conv::WgradTile<NI>;
-    const int itiles = (a.Cin + NI - 1) / NI, otiles = (a.Cout + mtb::conv::WG_OC - 1) / mtb::conv::WG_OC;
-    const int C32 = otiles * mtb::conv::WG_OC;
-    a.nblk = (int)((a.im.total() + mtb::conv::WG_PIX - 1) / mtb::conv::WG_PIX);
-    // two CTAs per SM (one where the tile's tensor memory allows no more)
-    const long long want = ((NI > 64 ? 148 : 296) + (long long)itiles * otiles - 1) / ((long long)itiles * otiles);
-    a.blk_per_split = (int)std::max<long long>(1, (a.nblk + want - 1) / want);
-    const int splits = (a.nblk + a.blk_per_split - 1) / a.blk_per_split;
-    const size_t off_b = align256((size_t)splits * 9 * a.Cin * C32 * sizeof(float));
-    const size_t off_s = off_b + align256((size_t)splits * C32 * sizeof(float));
-    Workspace& ws = workspace(off_s + (size_t)splits * ((a.Cin + 31) / 32) * sizeof(unsigned));
+    const int C32 = p.otiles * mtb::conv::WG_OC;
+    a.nblk = p.nblk;
+    a.blk_per_split = p.blk_per_split;
+    const size_t off_b = align256((size_t)p.splits * 9 * a.Cin * C32 * sizeof(float));
+    const size_t off_s = off_b + align256((size_t)p.splits * C32 * sizeof(float));
+    Workspace& ws = workspace(off_s + (size_t)p.splits * ((a.Cin + 31) / 32) * sizeof(unsigned));
     a.part = reinterpret_cast<float*>(ws.p);
     a.bpart = reinterpret_cast<float*>(ws.p + off_b);
     a.special = reinterpret_cast<unsigned*>(ws.p + off_s);
@@ -249,9 +273,9 @@ void wgrad_launch(mtb::conv::WgradArgs a, float* dw, float* db, cudaStream_t st)
     auto kern = mtb::conv::wgrad_kernel<NI>;
     const size_t smem = T::smem(a.im.W);
     MTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
-    mtb::launch_early(true, kern, dim3((unsigned)splits, (unsigned)itiles, (unsigned)otiles), mtb::conv::THREADS, smem, st, a);
-    mtb::launch_early(true, mtb::conv::wgrad_finalize_kernel, dim3((unsigned)otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st, a, splits,
-                      dw, db);
+    mtb::launch_early(true, kern, dim3((unsigned)p.splits, (unsigned)p.itiles, (unsigned)p.otiles), mtb::conv::THREADS, smem, st, a);
+    mtb::launch_early(true, mtb::conv::wgrad_finalize_kernel, dim3((unsigned)p.otiles, (unsigned)(a.Cin + 1), 3), 256, 0, st, a,
+                      p.splits, dw, db);
 }
 
 }  // namespace
@@ -295,12 +319,31 @@ mt_status mt_sg_conv3x3_backward_weight(const void* in, const void* dout, const 
         a.Cin = Cin;
         a.Cout = Cout;
         a.wait_ns = kWaitNs;
-        // input channels per CTA: the gradient tile is gathered once for each, so as many as the
-        // layer has and two stages of shared memory hold
-        if (Cin <= 16) wgrad_launch<16>(a, dw, db, st);
-        else if (Cin <= 32) wgrad_launch<32>(a, dw, db, st);
-        else if (Cin <= 64 || mtb::conv::WgradTile<128>::smem(W) > (size_t)kSmemMax) wgrad_launch<64>(a, dw, db, st);
-        else wgrad_launch<128>(a, dw, db, st);
+        const WgradPlan p = wgrad_plan(a.im, Cin, Cout);
+        switch (p.ni) {
+            case 16: wgrad_launch<16>(a, p, dw, db, st); break;
+            case 32: wgrad_launch<32>(a, p, dw, db, st); break;
+            case 64: wgrad_launch<64>(a, p, dw, db, st); break;
+            default: wgrad_launch<128>(a, p, dw, db, st); break;
+        }
+    });
+}
+
+mt_status mt_sg_conv3x3_plan(int B, int Cin, int Cout, int H, int W, int pass, int* plan) {
+    return run([&] {
+        check_shape(B, Cin, Cout, H, W);
+        if (pass < 0 || pass > 2 || !plan) mtb::fail(MT_ERR_INVALID_ARG, "bad plan arguments");
+        const mtb::conv::Image im = mtb::conv::image(B, H, W);
+        if (pass == 2) {
+            const WgradPlan p = wgrad_plan(im, Cin, Cout);
+            const int v[5] = {p.ni, 1, p.splits, p.blk_per_split, mtb::conv::WgradTile<16>::seg(W) != W + 1};
+            std::copy(v, v + 5, plan);
+        } else {
+            const ConvPlan p = pass ? conv_plan(im, Cout, Cin) : conv_plan(im, Cin, Cout);
+            const int seg = p.two ? mtb::conv::ConvTile<16, 2>::seg(W) : mtb::conv::ConvTile<16, 1>::seg(W);
+            const int v[5] = {p.bn, p.two ? 2 : 1, p.ksplit, p.blocks, seg != W + 1};
+            std::copy(v, v + 5, plan);
+        }
     });
 }
 

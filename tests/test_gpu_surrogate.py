@@ -61,8 +61,7 @@ def test_conv3x3_forward_and_gradients_match_torch(B, Cin, Cout, H, W):
 
 
 # tile edges of the implicit GEMM: rows around the 128- and 256-pixel tiles (one band of pixels or three
-# segments), one and two pixel tiles per CTA, 16/32/64 output channels, channels that are no multiple
-# of 8, 16 or 32, and clusters that share the input channels unevenly
+# segments), channels that are no multiple of 8, 16 or 32, and clusters that share the input channels unevenly
 @pytest.mark.parametrize("B,Cin,Cout,H,W", [(1, 40, 24, 3, 127), (1, 33, 40, 2, 130), (1, 16, 70, 1, 257), (2, 4, 3, 3, 600),
                                              (1, 300, 33, 4, 9), (1, 96, 256, 4, 4), (3, 1, 1, 1, 1), (20, 8, 40, 64, 64),
                                              (20, 9, 2, 64, 63), (20, 40, 32, 63, 64), (2, 130, 64, 5, 129)])
@@ -92,6 +91,38 @@ def test_weight_gradient_with_infinite_and_nan_inputs():
     ok = ref.isfinite()
     assert ok.any() and not ok.all()
     assert _rel(dw[ok], ref[ok]) < 1e-4
+
+
+# how mt_sg_conv3x3_plan cuts each shape: forward, data gradient (channels per CTA, pixel tiles, CTAs per sum, K blocks per
+# CTA, segments) and weight gradient. From three blocks per CTA on, a stage of shared memory is used again.
+PLANS = {(16, 32, 32, 64, 64): ((32, 1, 1, 1, 0), (32, 1, 1, 1, 0), (32, 1, 265, 2, 0)),
+         (8, 256, 64, 64, 64): ((64, 1, 1, 8, 0), (64, 1, 1, 2, 0), (128, 1, 34, 8, 0)),
+         (32, 256, 128, 12, 12): ((64, 1, 4, 2, 0), (64, 1, 2, 2, 0), (128, 1, 15, 3, 0)),
+         (64, 8, 16, 4, 300): ((16, 2, 1, 1, 1), (16, 2, 1, 1, 1), (16, 1, 251, 3, 1)),
+         (16, 160, 64, 64, 64): ((64, 1, 1, 5, 0), (64, 2, 1, 2, 0), (128, 1, 36, 15, 0)),
+         (16, 72, 40, 8, 300): ((64, 1, 1, 3, 1), (64, 2, 1, 2, 1), (64, 1, 68, 5, 1)),
+         (4, 512, 64, 40, 40): ((64, 1, 4, 4, 0), (64, 1, 1, 2, 0), (128, 1, 18, 3, 0)),
+         (1, 800, 16, 24, 24): ((16, 1, 8, 4, 0), (16, 1, 1, 1, 0), (128, 1, 5, 1, 0)),
+         (1, 300, 200, 9, 31): ((32, 1, 8, 2, 0), (16, 1, 4, 2, 0), (128, 1, 3, 1, 0)),
+         (8, 96, 64, 130, 130): ((64, 2, 1, 3, 0), (64, 2, 1, 2, 0), (64, 1, 72, 15, 1)),
+         (5, 36, 64, 100, 260): ((64, 2, 1, 2, 1), (64, 2, 1, 2, 1), (64, 1, 148, 7, 1)),
+         (2, 520, 48, 16, 140): ((64, 1, 4, 5, 1), (64, 1, 1, 2, 1), (64, 1, 13, 3, 1)),
+         (40, 32, 48, 64, 64): ((64, 2, 1, 1, 0), (32, 2, 1, 2, 0), (32, 1, 147, 9, 0)),
+         (30, 100, 20, 64, 64): ((32, 2, 1, 4, 0), (64, 2, 1, 1, 0), (128, 1, 142, 7, 0)),
+         (16, 200, 24, 10, 300): ((32, 1, 1, 7, 1), (64, 2, 1, 1, 1), (64, 1, 69, 6, 1))}
+
+
+@pytest.mark.parametrize("shape", PLANS)
+def test_conv3x3_on_every_way_of_cutting(shape):
+    """Every tile width with one and two pixel tiles, sums shared by up to eight CTAs, stages used again, bands and segments:
+    the plans are those listed, together with their results against torch."""
+    lib = capi.load()
+    B, Cin, Cout, H, W = shape
+    for k, want in enumerate(PLANS[shape]):
+        plan = (C.c_int * 5)()
+        capi.check(lib.mt_sg_conv3x3_plan(B, Cin, Cout, H, W, k, plan))
+        assert tuple(plan) == want, (k, tuple(plan))
+    test_conv3x3_forward_and_gradients_match_torch(*shape)
 
 
 @pytest.mark.parametrize("at", [(0, 0, 0), (0, 0, 5), (0, 4, 0), (1, 0, 0), (1, 4, 5), (1, 2, 3)])
