@@ -1,6 +1,8 @@
-"""run_confs replays each configuration as a CUDA graph (MTB_GRAPH, on by default), and run_prepared
-runs a range of prepared configurations as one graph: the captured launches are the ones issued
-directly, so results must be bit-identical to MTB_GRAPH=0, with the same launch count and progress.
+"""run_confs launches each configuration (batch) directly the first time, captures the second run of a launch sequence as a
+CUDA graph and replays it from then on (MTB_GRAPH, on by default), and run_prepared runs a range of
+prepared configurations as one graph: the captured launches are the ones issued directly, so results
+must be bit-identical to MTB_GRAPH=0, with the same launch count and progress, over the direct, the capturing and
+the replaying run of one engine.
 Cases: STEM with several probe batches and phonon configurations (the two configuration slots
 alternate, and the graphs replay), multiple output thicknesses, a tilted beam, exit waves, and the
 512^2 benchmark grid with full 256-probe batches."""
@@ -17,10 +19,13 @@ def _run(p, graph, monkeypatch, batch=8):
     monkeypatch.setenv("MTB_BATCH", str(batch))
     monkeypatch.setenv("MTB_PIPE", "3")  # no autotuner launches (they happen once per process and shape)
     e = api.Engine(p)
-    r = e.run()
-    n = e.launch_count()
+    r, n = [], []
+    for _ in range(4):  # both slots direct, captured, replayed with new contents, replayed
+        r.append(e.run())
+        n.append(e.launch_count())
     e.close()
-    return r, n
+    assert len(set(n)) == 1
+    return r, n[0]
 
 
 def _cases():
@@ -46,9 +51,10 @@ def test_graph_replay_is_bit_identical(name, monkeypatch):
     direct, n0 = _run(p, 0, monkeypatch, batch)
     graph, n1 = _run(p, 1, monkeypatch, batch)
     assert n1 == n0 > 0
-    for d0, d1 in zip(direct["data"], graph["data"]):
-        for k in d0:
-            np.testing.assert_array_equal(np.asarray(d1[k]), np.asarray(d0[k]), err_msg=k)
+    for run in graph + direct[1:]:
+        for d0, d1 in zip(direct[0]["data"], run["data"]):
+            for k in d0:
+                np.testing.assert_array_equal(np.asarray(d1[k]), np.asarray(d0[k]), err_msg=k)
 
 
 def test_prepared_range_runs_as_one_graph(monkeypatch):

@@ -7,7 +7,7 @@ real- and Fourier-space exit waves with a tilted beam, several thicknesses, the 
 electron diffraction with the coherent contribution, an HRTEM image with it, and displacements
 drawn on the GPU; over batches that
 divide the configurations and batches that do not (11 configurations: 8 + 3); through the graphs
-of mt_multislice_run and through direct launches (tests/test_gpu_batch.py covers the recorded runs
+of an engine run several times and through direct launches (tests/test_gpu_batch.py covers the recorded runs
 of mt_multislice_run_batch)."""
 import numpy as np
 import pytest
@@ -48,6 +48,13 @@ def test_batched_configurations_match_one_at_a_time(name, nconf, monkeypatch):
     assert got.keys() == ref.keys()
     for k in ref:
         np.testing.assert_array_equal(got[k], ref[k], err_msg=k)
+    # a kept engine launches its first run directly, captures its second and replays it
+    e = api.Engine(p)
+    for run in range(4):
+        got = _arrays(e.run())
+        for k in ref:
+            np.testing.assert_array_equal(got[k], ref[k], err_msg=f"{k}, run {run}")
+    e.close()
     # direct launches (no graphs) give the same
     monkeypatch.setenv("MTB_GRAPH", "0")
     direct = _arrays(api.ilc_multem(None, p))
