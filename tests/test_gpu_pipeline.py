@@ -60,15 +60,28 @@ def test_exit_wave_pipelined_matches_per_thread_kernels(nx, monkeypatch):
     np.testing.assert_array_equal(out[3], out[0])
 
 
-@pytest.mark.parametrize("shape", [1, 2])
-@pytest.mark.parametrize("nx", [64, 128, 256, 384, 512, 1024, 2048])
-def test_alternative_pipeline_shapes_match(nx, shape, monkeypatch):
-    """The autotuner's alternative pipeline shapes of the slice step (shape 1: columns owned by
-    warps at 256 and 512; shape 2: early issue with full exchange buffers, rows of 256 and 2048, columns of
-    384 and 1024) give the waves of the per-thread-load kernels bit for bit."""
-    p = specimens.stem_srtio3(nx=nx, ny=nx, na=4, nb=4, nc=6 if nx < 2048 else 2, ns=4, nconf=1, seed=3)
+# the lengths that have an alternative shape; probes so that every group of every CTA takes several tiles or units, with and
+# without a remainder (columns of 256: 32 tiles of 8 columns per probe over 148 CTAs of six groups; rows of 256 take
+# whole groups of eight probes), and other line lengths in the other direction, which set the strides
+@pytest.mark.parametrize("nx,ny,shape,ns", [(256, 256, 1 << 2, 4), (256, 256, 1 << 2, 8), (256, 256, 1 << 2, 9), (256, 512, 1 << 2, 7),
+                                            (256, 64, 1 << 2, 16), (512, 512, 1 << 2, 4), (512, 512, 1 << 2, 7), (512, 128, 1 << 2, 9),
+                                            (512, 1024, 1 << 2, 5), (256, 256, 2, 8), (256, 256, 2, 4), (128, 256, 2, 8),
+                                            (2048, 2048, 2, 4), (64, 2048, 2, 4), (384, 384, 2 << 2, 4), (384, 384, 2 << 2, 7),
+                                            (384, 256, 2 << 2, 8), (1024, 1024, 2 << 2, 4), (1024, 256, 2 << 2, 5)])
+def test_alternative_pipeline_shapes_match(nx, ny, shape, ns, monkeypatch):
+    """The autotuner's alternative pipeline shapes of the slice step (columns, bits 2-3: 1 owned by warps at 256 and 512, 2
+    early issue with full exchange buffers at 384 and 1024; rows, bits 0-1: 2 the same at 256 and 2048) give the
+    waves of the per-thread-load kernels bit for bit."""
+    p = specimens.stem_srtio3(nx=nx, ny=ny, na=4, nb=4, nc=6 if max(nx, ny) < 2048 else 2, ns=ns, nconf=1, seed=3)
+    monkeypatch.setenv("MTB_BATCH", str(ns * ns))
     ref = _stem(p, 0, monkeypatch)
-    monkeypatch.setenv("MTB_SHAPE", str(shape | (shape << 2)))
+    monkeypatch.setenv("MTB_SHAPE", str(shape))
+    monkeypatch.setenv("MTB_PIPE", "3")
+    e = api.Engine(p)
+    e.run()
+    t = e.tuning()
+    e.close()
+    assert t["probes_per_launch"] == ns * ns and (t["cols"] == 1 + (shape >> 2) if shape > 3 else t["rows"] == 1 + shape), t
     img = _stem(p, 3, monkeypatch)
     monkeypatch.delenv("MTB_SHAPE")
     if nx == 1024:
