@@ -95,13 +95,6 @@ struct AtomFoot {
     int type, pad;
 };
 
-// Spline tables in shared memory: per type nR knot pairs (R2[i], R2[i+1]) and coefficients (c0..c3)[i].
-struct SplatTables {
-    const float2* knot;
-    const float4* coef;
-    int nR;
-};
-
 __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
     unsigned long long d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -133,7 +126,7 @@ __device__ __forceinline__ float spline_interval(const float2* knot, int nR, flo
 
 template <int PX>
 __global__ void __launch_bounds__(SPLAT_THREADS) splat_kernel(SplatArgs a, int islice_0, int n_slice) {
-    extern __shared__ float4 sm_coef[];  // n_types * nR coefficients, then the knot pairs
+    extern __shared__ float4 sm_coef[];  // n_types * nR coefficients (c0..c3)[i], then the knot pairs (R2[i], R2[i+1])
     __shared__ AtomFoot s_list[SPLAT_THREADS];
     __shared__ int s_warp_cnt[SPLAT_WARPS];
     __shared__ float2 s_guess[kMaxTypes];  // log2(R2) -> interval: scale, offset

@@ -436,7 +436,7 @@ struct RowPipe {
     static constexpr size_t SMEM = sizeof(float2) * (TW + LAND + NG * SLOT + NG * HBUF);
     static constexpr bool OK = (GT % TPL == 0) && (GT % 32 == 0) && (SLOT % 2 == 0) && (HBUF % 2 == 0) &&
                                (TW % 2 == 0) &&
-                               SMEM <= kPipeSmemMax && (GT == 32 || NG <= 14) &&
+                               SMEM <= kPipeSmemMax && NG <= 14 &&
                                (PM != 1 || (HalfExchange<NY, false>::OK && HalfExchange<NY, true>::OK));
 };
 
@@ -520,8 +520,7 @@ __global__ void __launch_bounds__(GT * NG, 1) rows_pipe_kernel(RowArgs a) {
     }
 
     using Sync = typename std::conditional<(TPL <= 32), WarpSync, GroupSync<GT>>::type;
-    using GSync = typename std::conditional<(GT == 32), WarpSync, GroupSync<GT>>::type;
-    const GSync gsync{grp};
+    const GroupSync<GT> gsync{grp};
     for (int k = grp; k < K; k += NG) {
         const long long item = i0 + k;
         const int g = (int)(item / a.nprobe), b = (int)(item % a.nprobe);
@@ -617,7 +616,6 @@ struct RowPipeShape<NY, 2> {
 template <int NX, int GT, int NG, int PM = (HalfExchange<NX, false>::OK && HalfExchange<NX, true>::OK) ? 1 : 0, bool OWN = false>
 struct ColPipe {
     using G = LineGeom<NX>;
-    static constexpr int PM_V = PM;
     static constexpr bool EARLY = PM != 0;
     static constexpr int W = GT / G::TPL;
     static constexpr int LSH = PM == 1 ? HalfLineSmem<NX>::value : col_ls<NX, W>();  // exchange buffer per column
@@ -635,7 +633,7 @@ struct ColPipe {
                                (BOXR > 0) && (NX % (BOXR > 0 ? BOXR : 1) == 0) && ((size_t)NX * W <= LAND) &&
                                (((TW + NX) * sizeof(float2)) % 128 == 0) &&
                                (GT % G::TPL == 0) && (GT % 32 == 0) && (W % 2 == 0) && (2 * W <= 256) &&
-                               (HBUF % 2 == 0) && SMEM <= kPipeSmemMax && (GT == 32 || NG <= 14);
+                               (HBUF % 2 == 0) && SMEM <= kPipeSmemMax && NG <= 14;
 };
 
 // Column-pass pipeline shapes: 2 groups of 256 threads (default), and the alternatives the autotuner
@@ -706,7 +704,7 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     const int grp = threadIdx.x / GT, gtid = threadIdx.x % GT;
     const int cs = gtid % W, ts = gtid / W;  // column and line thread that this thread stores
     const int c = OWN ? gtid / G::TPL : cs, t = OWN ? gtid % G::TPL : ts;  // ... and transforms
-    static_assert(!OWN || (ColOwn<NX, GT, PM>::OK && INV), "whole-line ownership needs a swizzled tile and an inverse");
+    static_assert(!OWN || (ColOwn<NX, GT, PM>::OK && INV && EARLY), "whole-line ownership needs a swizzled tile of its own and an inverse");
     float2* land = land0 + grp * P::LAND;
     float2* buf = EARLY ? land0 + NG * P::LAND + grp * P::HBUF + (size_t)c * P::LSH : land + (size_t)c * P::LSH;
     (void)HALF;
@@ -743,9 +741,8 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
     };
     if (gtid == 0 && grp < K) issue(grp);
 
-    using GSync = typename std::conditional<(GT == 32), WarpSync, GroupSync<GT>>::type;
-    using FSync = typename std::conditional<OWN, WarpSync, GSync>::type;
-    const GSync gsync{grp};
+    using FSync = typename std::conditional<OWN, WarpSync, GroupSync<GT>>::type;
+    const GroupSync<GT> gsync{grp};
     const FSync fsync{grp};
     for (int k = grp; k < K; k += NG) {
         const int item = items - 1 - (int)(blockIdx.x + k * gridDim.x);  // the last wave first (see cols_launch_ld)
@@ -795,10 +792,6 @@ __global__ void __launch_bounds__(GT * NG, 1) cols_pipe_kernel(ColArgs a, const 
         if constexpr (INV) {
             if constexpr (OWN) {
                 line_fft_owner<NX, true, +1, HALF>(x, buf, t, buf + (ptrdiff_t)(cs - c) * P::LSH, ts, twR, gsync);
-                if constexpr (!EARLY) {
-                    gsync();  // every exchange read of the slot is done
-                    if (gtid == 0 && k + NG < K) issue(k + NG);
-                }
             } else if constexpr (HALF) {
                 line_fft_half<NX, true, +1>(x, buf, twR, t, gsync);
             } else {
