@@ -465,12 +465,12 @@ def run_ours(args):
     achieved = bytes_per_launch / (avg / 1e3) / 1e9
     prof = profile_traffic()
     traffic = None
-    if prof and dom in prof:
+    if prof and dom in prof and prof[dom].get("variant") == eng.tuning()[dom]:  # captured on the variant that ran
         traffic = prof[dom].get("dram_bytes_per_launch_scaled")
     eng.close()  # its device memory returns to the library's pool, which the next engine reuses
 
     if rank == 0:
-        # end to end through the public C ABI: host input struct -> mt_multislice_run -> host output
+        # end to end through the public API: host input -> api.ilc_multem -> host output
         ke = max(1, min(K, 2))
         pe = workload(ke, seed=5)
         api.ilc_multem(conf, workload(1, seed=4))  # untimed warm-up call
@@ -501,7 +501,7 @@ def run_ours(args):
                                               "cols": "bulk-copy fed" if variants & 2 else "per-thread loads"}},
                "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                        "steps": ke, "calls_s": [round(c, 4) for c in calls],
-                       "api": "mt_multislice_run (C ABI), host in/out, includes engine set-up; median of 3 calls "
+                       "api": "api.ilc_multem (mt_multislice_run_rows of the C ABI), host in/out, includes engine set-up; median of 3 calls "
                               "after one warm-up call"},
                "gpu_launches": launches,
                "clocks": clk.summary()}
