@@ -379,7 +379,7 @@ def uneven_batch_live(conf):
 
 def large_field_live(conf):
     """Exit wave of 2 nm amorphous carbon on Au(110) 12x17x60 cells on a 2048^2 grid (200 kV, 2 A
-    slices), 8 phonons, through mt_multislice_run after one warm-up call."""
+    slices), 8 phonons, through api.ilc_multem after one warm-up call."""
     from multem_b200 import api, specimens
     api.ilc_multem(conf, specimens.au110_amorphous_carbon(nconf=1))
     p = specimens.au110_amorphous_carbon(nconf=8)
@@ -390,7 +390,7 @@ def large_field_live(conf):
     return {"workload": "2 nm a-C on Au(110) 12x17x60 cells (29,292 atoms), 2048^2, 200 kV, 2 A slices, 8 phonons, "
                         "exit wave (EWRS)", "slices": n_sl, "seconds": dt,
             "slice_updates_per_s": 8 * n_sl / dt,
-            "api": "mt_multislice_run (host in/out, set-up included)"}
+            "api": "api.ilc_multem (host in/out, set-up included)"}
 
 
 def run_profile_case(args):

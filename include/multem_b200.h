@@ -280,7 +280,8 @@ mt_status mt_engine_run_rows(mt_engine* eng, mt_output_multislice* out);
  * their weighted detector sums into the engine's FP64 accumulators without writing output. Used to
  * shard configurations over GPUs; mt_engine_read_stem() then returns the partial sums. */
 mt_status mt_engine_run_confs(mt_engine* eng, int iconf_0, int iconf_e);
-/* Zero the engine's accumulators. */
+/* Zero the engine's accumulators. Queued on the engine's stream: the call does not wait for the device, and what is
+ * run or read afterwards comes after it. */
 mt_status mt_engine_reset(mt_engine* eng);
 /* STEM: copy the FP64 accumulators image_tot[ithk][idet][ny*nx] to host memory. */
 mt_status mt_engine_read_stem(mt_engine* eng, double* image_tot, size_t n);

@@ -67,7 +67,8 @@ class OutputBuffers:
         self.c = o
 
     def rows_to_dict(self):
-        """Output dict of a run that wrote row-major images (mt_*_run_rows): they are the arrays."""
+        """Output dict of a run that wrote row-major images (mt_*_run_rows). Its arrays are views of one buffer per quantity
+        (all thicknesses and detectors), which lives as long as any of them: copy an image to keep it alone."""
         d = self.d
         nt, nd, nx, ny = d.n_thick, d.n_detector, d.nx, d.ny
         res = {"dx": self.c.dx, "dy": self.c.dy, "x": self.x[:d.n_x], "y": self.y[:d.n_y], "thick": self.thick[:nt],

@@ -353,8 +353,8 @@ struct ConvTile {
 // Bound by the chain of a CTA (about 18 k cycles: weights 3 k, gather 2-5 k, the MMAs' reads of the pixel
 // operand, 40 cycles each with 32 channels, epilogue 3 k, or 7-10 k over a cluster), which three CTAs
 // per SM overlap (two: 44 us, four: 37 us for the first layer below). Measured on one B200: 16 images of
-// 32 -> 32 channels at 128 x 128, forward 39 us and data gradient 43 us (im2col through memory and a
-// GEMM: 205 us each); 32 images of 256 -> 256 channels at 4 x 4, forward 15 us.
+// 32 -> 32 channels at 128 x 128, forward 32 us and data gradient 36 us (im2col through memory and a
+// GEMM: 205 us each); 32 images of 256 -> 256 channels at 4 x 4, forward 13 us, data gradient 13 us.
 template <int BN, int MT, bool DGRAD>
 __global__ void __launch_bounds__(THREADS, 3) conv_kernel(const ConvArgs a) {
     using T = ConvTile<BN, MT>;
@@ -584,8 +584,8 @@ struct WgradTile {
 // sums per split, added in split order by wgrad_finalize_kernel. The zeros between rows and images
 // take part in the products, so an infinite or NaN input beside them would reach taps that it has no
 // part in: such channels are noted for the split (WgradArgs::special) and their sums taken without the padding.
-// 16 images of 32 -> 32 channels at 128 x 128: 53 us and 8 us for the finalize kernel (transposed im2col,
-// GEMM and finalize through memory: 195 us).
+// 16 images of 32 -> 32 channels at 128 x 128: 55 us with the finalize kernel (transposed im2col, GEMM and
+// finalize through memory: 195 us).
 template <int NI>
 __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradArgs a) {
     using T = WgradTile<NI>;
