@@ -5,7 +5,6 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
-#include <thread>
 #include <vector>
 #include <exception>
 #include <memory>
@@ -14,6 +13,7 @@
 #include "common.hpp"
 #include "devmem.hpp"
 #include "engine.hpp"
+#include "host_threads.hpp"
 #include "matio.hpp"
 #include "multem_b200.h"
 
@@ -328,12 +328,7 @@ static bool run_batch_graph(const mt_system_conf& c, int n, const mt_input_multi
             if (st[i] != MT_OK) msg[i] = g_last_error;
         }
     };
-    {
-        std::vector<std::thread> pool;
-        for (int t = 1; t < workers; t++) pool.emplace_back(build);
-        build();
-        for (auto& t : pool) t.join();
-    }
+    mtb::run_threads(workers, [&](int) { build(); });
     if (oom) {  // the engines are released here; the host-worker path runs the batch
         for (int i = 0; i < n; i++) {
             st[i] = MT_OK;
@@ -440,10 +435,7 @@ mt_status mt_multislice_run_batch(const mt_system_conf* conf, int n, const mt_in
                 if (st[i] != MT_OK) msg[i] = g_last_error;
             }
         };
-        std::vector<std::thread> pool;
-        for (int t = 1; t < workers; t++) pool.emplace_back(work);
-        work();
-        for (auto& t : pool) t.join();
+        mtb::run_threads(workers, [&](int) { work(); });
         for (int i = 0; i < n; i++)
             if (st[i] != MT_OK) throw mtb::Error(st[i], "input " + std::to_string(i) + ": " + msg[i]);
     });

@@ -65,3 +65,9 @@ def test_parts_run_once_whatever_fails(tmp_path):
     (tmp_path / "t.cpp").write_text("#include <string>\n" + PROGRAM)
     subprocess.run([gxx, "-std=c++17", "-O1", "-pthread", f"-I{CSRC}", "-o", tmp_path / "t", tmp_path / "t.cpp"], check=True)
     assert subprocess.run([tmp_path / "t"], timeout=60).returncode == 0
+
+
+def test_threads_are_started_nowhere_else():
+    """A std::thread of its own would end the process where an exception passes it by."""
+    for f in CSRC.glob("*.c*"):
+        assert "std::thread>" not in f.read_text() and "std::thread " not in f.read_text(), f.name
